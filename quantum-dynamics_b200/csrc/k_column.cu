@@ -1,4 +1,6 @@
-// k_column.cu -- the column pass of one split-operator step, SIMT form.
+// k_column.cu -- the column pass of one split-operator step, SIMT form (the
+// complex64 form where the tensor-core kernel is not built, and the FP64 form of
+// bases that k_column_dmma.cu does not hold in shared memory).
 //
 // For a tile of TP grid columns (R_i, r_j) it performs, in shared memory,
 //   psi_theta = B psi_l                    BackwardLegendreTransform (LegTransform.F:34-59)
@@ -176,6 +178,7 @@ template <typename R>
 cudaError_t launch_column(const ColumnParams &p, int mode, cudaStream_t s)
 {
   typedef typename Cplx<R>::T C;
+  if (sizeof(R) == 8 && column_dmma_ok(p.nth, p.nl)) return launch_column_dmma(p, mode, s);
   int TP = 32;
   while (TP > 8 && (size_t)(p.nl + p.nth) * TP * sizeof(C) > 96 * 1024) TP /= 2;
   const size_t sm = (size_t)(p.nl + p.nth) * TP * sizeof(C) + 32 * sizeof(double);

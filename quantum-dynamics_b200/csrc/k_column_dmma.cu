@@ -1,0 +1,374 @@
+// k_column_dmma.cu -- the FP64 column pass on the FP64 tensor cores.
+//
+// Per tile of 16 grid columns, the work of k_column.cu (B, absorber, surface
+// rows, norm, exp(-iVdt), F) as two GEMMs of mma.sync m16n8k8 .f64.  One
+// 16-row operand holds eight grid columns: rows 0-7 their real parts, rows
+// 8-15 their imaginary parts, so the thread that gets an accumulator's real
+// value also gets its imaginary one and the theta-space work needs no exchange.
+//   GEMM1  psi_theta[col][k] = sum_l psi_l[col][l] P[k][l]
+//   GEMM2  psi_l[col][l] = (l + 1/2) sum_k (w_k psi_theta[col][k]) P[k][l]
+// Both read ONE copy of P (n_theta x n_l, 128 KB at 128 x 128), which stays in
+// shared memory while the CTA walks its tiles: w_k is applied to the
+// theta-space values and l + 1/2 to the results (two copies, P and (l+1/2) w P,
+// would not fit).  The contraction index of an mma may be permuted freely: slot
+// (t, i) takes index 2t + i, so GEMM1's operand of P is one 16-byte load.
+//
+// Bound: FP64 tensor throughput (measured 37.0 TFLOP/s for back-to-back
+// m16n8k8, one warp per scheduler or more; plain DFMA chains 34).  FP64
+// operands need 8 x 8 values in registers per thread to keep plain FMAs fed
+// from shared memory; with mma the warps of an SM read about 64 B a clock.
+// Tile of 16 columns, not 32: two tiles' buffers (the next one arrives by
+// cp.async while this one is multiplied) fit beside P at 128 x 128, and grids
+// of a few hundred tiles spread over the SMs.  Per launch, against the SIMT
+// kernel: 256 x 192 x 128 (6.4 GFLOP) 835 -> 258 us, 128 x 128 x 64 87 -> 35 us,
+// 64 x 64 x 40 30 -> 13 us (each with 5 us of event and launch time).
+//
+// Shared layouts: a tile is [row][17] complex (17: every 16-byte access of a
+// warp touches the eight bank groups evenly); P is [k][nlp], nlp a multiple of
+// 16, with the 16-byte units of row k permuted by XOR (swz) so that both the
+// pair loads along l (GEMM1) and the loads down k (GEMM2) are free of conflicts.
+#include "qd_kernels.h"
+
+namespace {
+
+constexpr int TC = 16;          // grid columns of a tile
+constexpr int LD = TC + 1;      // tile row stride (complex)
+constexpr int MAXGRP = 16;      // groups of eight angles or orders
+
+__device__ __forceinline__ void dmma(double (&c)[4], const double2 a0, const double2 a1,
+                                     double b0, double b1)
+{
+  asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%0,%1,%2,%3};"
+      : "+d"(c[0]), "+d"(c[1]), "+d"(c[2]), "+d"(c[3])
+      : "d"(a0.x), "d"(a0.y), "d"(a1.x), "d"(a1.y), "d"(b0), "d"(b1));
+}
+
+// permutation of the 16-byte units of row k of P, within groups of eight
+__device__ __forceinline__ int swz(int k) { return ((k & 1) << 2) ^ (((k >> 1) & 3) << 1); }
+
+__device__ __forceinline__ void cp16(void *dst, const void *src, bool valid)
+{
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  const int n = valid ? 16 : 0;                 // 0: fill the 16 bytes with zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(d), "l"(src), "r"(n)
+               : "memory");
+}
+
+__host__ __device__ inline int pad8(int n) { return (n + 7) & ~7; }
+__host__ __device__ inline int pad16(int n) { return (n + 15) & ~15; }
+inline size_t dmma_smem(int nth, int nl)
+{
+  const size_t rows = pad8(nth) > pad8(nl) ? pad8(nth) : pad8(nl);
+  return sizeof(double) * (size_t)pad8(nth) * pad16(nl) + 2 * sizeof(double2) * rows * LD +
+         sizeof(double) * pad8(nth);
+}
+
+// acc[m][n] = tile (columns 8 m + g) x P over kb blocks of 8 contraction
+// indices; the warp's n-th output group: rows 8 (wn + WN n) + ... of the result.
+// The XOR of P's units changes with a block's parity only (GEMM1) or not at
+// all (GEMM2), so a lane's addresses advance by constants.
+template <int MI, int NI, int WN, bool FWD>
+__device__ __forceinline__ void gemm(double (&acc)[MI][NI][4], const double2 *tile, const double *P,
+                                     int nlp, int kb, int ngrp, int wn, int g, int t)
+{
+#pragma unroll
+  for (int m = 0; m < MI; m++)
+#pragma unroll
+    for (int n = 0; n < NI; n++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) acc[m][n][i] = 0.0;
+  const double2 *row = tile + 2 * t * LD + g;
+  const double *pk[NI];                 // FWD: P[2t][8 grp + g]; else P[8 grp + g][..]
+  int o0[NI], o1[NI];                   // FWD: rows 2t, 2t + 1; else even, odd block
+#pragma unroll
+  for (int n = 0; n < NI; n++) {
+    const int grp = wn + WN * n, k = FWD ? 2 * t : 8 * grp + g;
+    if (FWD) {
+      const int u = 4 * grp + (g >> 1);
+      pk[n] = P + (g & 1);
+      o0[n] = k * nlp + 2 * (u ^ swz(k));
+      o1[n] = (k + 1) * nlp + 2 * (u ^ swz(k + 1));
+    } else {
+      pk[n] = P + k * nlp;
+      o0[n] = 2 * (t ^ swz(k));
+      o1[n] = 2 * ((4 + t) ^ swz(k));
+    }
+  }
+  auto block = [&](int b) {
+    double2 a[MI][2];
+#pragma unroll
+    for (int m = 0; m < MI; m++) {
+      a[m][0] = row[8 * m];
+      a[m][1] = row[LD + 8 * m];
+    }
+    row += 8 * LD;
+#pragma unroll
+    for (int n = 0; n < NI; n++) {
+      if (wn + WN * n >= ngrp) break;             // the same for the whole warp
+      double b0, b1;
+      if (FWD) {                                  // P[8 b + 2t, + 1][8 grp + g]
+        b0 = pk[n][o0[n]];
+        b1 = pk[n][o1[n]];
+        pk[n] += 8 * nlp;
+      } else {                                    // P[8 grp + g][8 b + 2t, + 1]
+        const double2 v = *reinterpret_cast<const double2 *>(pk[n] + ((b & 1) ? o1[n] : o0[n]));
+        b0 = v.x;
+        b1 = v.y;
+        if (b & 1) pk[n] += 16;
+      }
+#pragma unroll
+      for (int m = 0; m < MI; m++) dmma(acc[m][n], a[m][0], a[m][1], b0, b1);
+    }
+  };
+  int b = 0;
+  for (; b + 4 <= kb; b += 4) {
+    block(0);
+    block(1);
+    block(2);
+    block(3);
+  }
+  for (; b < kb; b++) block(b);
+}
+
+// WM x WN warps: warp (wm, wn) takes 16 / WM of the tile's columns and every
+// WN-th group of eight outputs, NI of them
+template <int WM, int WN, int NI, int MODE>
+__global__ void __launch_bounds__(WM * WN * 32, 16 / (WM * WN)) k_column_dmma(ColumnParams p)
+{
+  constexpr int NT = WM * WN * 32, MI = 2 / WM;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int nthp = pad8(p.nth), nlp = pad16(p.nl), nl8 = pad8(p.nl);
+  const int rows = nthp > nl8 ? nthp : nl8;
+  double2 *buf = reinterpret_cast<double2 *>(smem);       // [2][rows][LD]
+  double *P = reinterpret_cast<double *>(buf + 2 * rows * LD);
+  double *w = P + nthp * nlp;
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int wn = (tid >> 5) % WN, c0 = 8 * MI * ((tid >> 5) / WN);   // the warp's first column
+  const int n12 = (int)p.n12;
+  const int tiles_per_run = (n12 + TC - 1) / TC;
+  const int kgrp = nthp >> 3, lgrp = nl8 >> 3;
+  pdl_trigger();
+
+  // tiles blockIdx.x, + gridDim.x, ...: position `at` of the runs' order, tile `in` of that run
+  struct Pos { int at, in; };
+  auto step = [&](Pos x) {
+    x.in += gridDim.x;
+    while (x.in >= tiles_per_run) {
+      x.in -= tiles_per_run;
+      x.at++;
+    }
+    return x;
+  };
+  auto run_of = [&](Pos x) { return p.run_order ? p.run_order[x.at] : x.at; };
+  auto load_P = [&](int set) {
+    const double *src = p.P + set * p.set_stride;
+    const int half = nlp >> 1;
+    for (int x = tid; x < nthp * half; x += NT) {
+      const int k = x / half, u = x - k * half, l = 2 * u;
+      const double *s = src + k * p.nl + l;
+      const bool in = k < p.nth;
+      reinterpret_cast<double2 *>(P)[k * half + (u ^ swz(k))] =
+          make_double2(in && l < p.nl ? __ldg(s) : 0.0, in && l + 1 < p.nl ? __ldg(s + 1) : 0.0);
+    }
+  };
+  // the l-space tile (MID, TAIL) into buffer b, rows past n_l and columns past the grid zero
+  auto fetch = [&](Pos x, int b) {
+    if (MODE != COL_HEAD && x.at < p.nruns) {
+      const int c = tid % TC, q = x.in * TC + c;
+      const double2 *src = reinterpret_cast<const double2 *>(p.lpsi) +
+                           (long)run_of(x) * p.nl * p.n12;
+      const double2 *s = src + (long)(tid / TC) * n12 + q;
+      double2 *d = buf + (b * rows + tid / TC) * LD + c;
+      for (int l = tid / TC; l < nl8; l += NT / TC, s += (long)(NT / TC) * n12, d += NT / TC * LD) {
+        const bool ok = l < p.nl && q < n12;
+        cp16(d, ok ? s : src, ok);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  for (int k = tid; k < nthp; k += NT) w[k] = k < p.nth ? p.w[k] : 0.0;
+  Pos pos = {(int)blockIdx.x / tiles_per_run, (int)blockIdx.x % tiles_per_run};
+  int run = run_of(pos), set = p.run_set ? p.run_set[run] : 0;
+  load_P(set);
+  pdl_wait();                                       // psi_l: the l-space pass's output
+  fetch(pos, 0);
+  double nsum = 0.0, esum = 0.0;
+  auto flush = [&](int r) {                         // this thread's sums over run r's tiles
+    for (int o = 16; o > 0; o >>= 1) {
+      nsum += __shfl_xor_sync(0xffffffffu, nsum, o);
+      esum += __shfl_xor_sync(0xffffffffu, esum, o);
+    }
+    if (lane == 0 && p.norm_out) atomicAdd(p.norm_out + r, nsum);
+    if (lane == 0 && p.esum) atomicAdd(p.esum + 3 * r + 2, esum);
+    nsum = esum = 0.0;
+  };
+
+  const int k0 = 8 * wn + 2 * t;                    // this thread's first angle and first order
+  Pos next;
+  for (int it = 0; pos.at < p.nruns; it++, pos = next) {
+    next = step(pos);
+    const int r = run_of(pos);
+    if (r != run) {
+      if (MODE != COL_HEAD) flush(run);
+      run = r;
+      const int s = p.run_set ? p.run_set[run] : 0;
+      if (s != set) {
+        __syncthreads();                            // the previous tile's reads of P are done
+        set = s;
+        load_P(set);
+      }
+    }
+    const int p0 = pos.in * TC;
+    const long zoff = (long)run * p.nth * p.n12, voff = (long)run * p.vrun;
+    double2 *cur = buf + (it & 1) * rows * LD;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                // the tile (and P) in place; the other buffer free
+    fetch(next, (it & 1) ^ 1);
+
+    double acc[MI][NI][4];
+    if (MODE != COL_HEAD) {
+      // exp(-iVdt) of this thread's values, in flight during GEMM1
+      double2 ph[MI][NI][2];
+      if (MODE == COL_MID) {
+#pragma unroll
+        for (int m = 0; m < MI; m++) {
+          const int q = p0 + c0 + 8 * m + g;
+          const double2 *v = p.expV + voff + (long)k0 * n12 + q;
+#pragma unroll
+          for (int n = 0; n < NI; n++)
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+              if (k0 + 8 * WN * n + i < p.nth && q < n12)
+                ph[m][n][i] = __ldg(v + (long)(8 * WN * n + i) * n12);
+        }
+      }
+      gemm<MI, NI, WN, false>(acc, cur + c0, P, nlp, lgrp, kgrp, wn, g, t);
+      __syncthreads();                              // every read of the l-space tile is done
+#pragma unroll
+      for (int m = 0; m < MI; m++) {
+        const int q = p0 + c0 + 8 * m + g;
+        const bool in = q < n12;
+        const int j = in ? q / p.n1 : 0, i1 = in ? q - j * p.n1 : 0;
+        const double d = in && p.d1 ? p.d1[i1] * p.d2[j] : 1.0;
+        const bool fl = in && p.do_flux && j >= p.surf_j0 && j < p.surf_j0 + p.surf_nrows;
+        double2 *surf = reinterpret_cast<double2 *>(p.surf) +
+                        ((long)run * p.surf_nrows + (fl ? j - p.surf_j0 : 0)) * p.nth * p.n1 + i1;
+#pragma unroll
+        for (int n = 0; n < NI; n++) {
+          if (wn + WN * n >= kgrp) break;
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const int k = k0 + 8 * WN * n + i;
+            double2 v = make_double2(acc[m][n][i], acc[m][n][2 + i]);
+            if (k < p.nth && in) {
+              const double wk = w[k];
+              if (p.esum)
+                esum += wk * (v.x * v.x + v.y * v.y) * p.pot[voff + (long)k * n12 + q];
+              v = cscale(v, d);
+              if (fl) surf[k * p.n1] = v;
+              nsum += wk * (v.x * v.x + v.y * v.y);
+              if (MODE == COL_TAIL && p.out_z) p.psi_z[zoff + (long)k * n12 + q] = v;
+              if (MODE == COL_MID) v = cscale(cmul(v, ph[m][n][i]), wk);
+            } else {
+              v = make_double2(0.0, 0.0);
+            }
+            if (MODE == COL_MID) cur[k * LD + c0 + 8 * m + g] = v;
+          }
+        }
+      }
+      if (MODE == COL_TAIL) continue;
+    } else {
+      for (int x = tid; x < nthp * TC; x += NT) {
+        const int k = x / TC, c = x % TC, q = p0 + c;
+        const long o = (long)k * n12 + q;
+        double2 z = make_double2(0.0, 0.0);
+        if (k < p.nth && q < n12) {
+          z = p.psi_z[zoff + o];
+          double s, co;
+          sincos(p.dt * p.pot[voff + o], &s, &co);  // exp(-i V dt) = (co, -s)
+          double2 f = make_double2(co, -s);
+          if (p.prestep) {
+            // psi / sqrt(v) * v = psi * sqrt(v), principal branch
+            // (pre_evolution_with_potential_dt_2, timeEvol.C:519-538)
+            double sh, ch;
+            sincos(0.5 * atan2(-s, co), &sh, &ch);
+            f = make_double2(ch, sh);
+          }
+          z = cscale(cmul(z, f), w[k]);
+        }
+        cur[k * LD + c] = z;
+      }
+    }
+    __syncthreads();                                // the theta-space tile in place
+    gemm<MI, NI, WN, true>(acc, cur + c0, P, nlp, kgrp, lgrp, wn, g, t);
+#pragma unroll
+    for (int m = 0; m < MI; m++) {
+      const int q = p0 + c0 + 8 * m + g;
+      if (q >= n12) continue;
+      double2 *dst = reinterpret_cast<double2 *>(p.lpsi) + ((long)run * p.nl + k0) * p.n12 + q;
+#pragma unroll
+      for (int n = 0; n < NI; n++)
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const int l = k0 + 8 * WN * n + i;
+          if (l < p.nl)
+            dst[(long)(8 * WN * n + i) * n12] =
+                make_double2((l + 0.5) * acc[m][n][i], (l + 0.5) * acc[m][n][2 + i]);
+        }
+    }
+  }
+  if (MODE != COL_HEAD) flush(run);
+}
+
+template <int WM, int WN, int NI, int MODE>
+cudaError_t launch(const ColumnParams &p, cudaStream_t s)
+{
+  const size_t sm = dmma_smem(p.nth, p.nl);
+  cudaError_t e = cudaFuncSetAttribute(k_column_dmma<WM, WN, NI, MODE>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  if (e != cudaSuccess) return e;
+  const long ntiles = (p.n12 + TC - 1) / TC * p.nruns;
+  const int by_regs = 16 / (WM * WN);
+  const long slots = 148L * (by_regs > 1 && sm <= 113 * 1024 ? by_regs : 1);   // CTAs resident at once
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(ntiles < slots ? ntiles : slots));
+  cfg.blockDim = dim3(WM * WN * 32);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, k_column_dmma<WM, WN, NI, MODE>, p);
+  return cudaGetLastError();
+}
+
+template <int WM, int WN, int NI>
+cudaError_t launch_mode(const ColumnParams &p, int mode, cudaStream_t s)
+{
+  switch (mode) {
+    case COL_HEAD: return launch<WM, WN, NI, COL_HEAD>(p, s);
+    case COL_MID: return launch<WM, WN, NI, COL_MID>(p, s);
+    default: return launch<WM, WN, NI, COL_TAIL>(p, s);
+  }
+}
+
+}  // namespace
+
+// P and two tiles in shared memory, and no more than MAXGRP groups on either side
+bool column_dmma_ok(int nth, int nl)
+{
+  return pad8(nth) <= 8 * MAXGRP && pad8(nl) <= 8 * MAXGRP && dmma_smem(nth, nl) <= 227 * 1024;
+}
+
+cudaError_t launch_column_dmma(const ColumnParams &p, int mode, cudaStream_t s)
+{
+  // 64 angles and orders or fewer: P and two tiles take 68 KB at most, two CTAs
+  // of 8 warps share an SM (128 x 128 x 64: 35.1 us a launch, 39.2 with one CTA of
+  // 16 warps); more: one CTA of 16 warps (256 x 192 x 128: 258 us, 275 with 8)
+  return pad8(p.nth) <= 64 && pad8(p.nl) <= 64 ? launch_mode<2, 4, 2>(p, mode, s)
+                                               : launch_mode<2, 8, 2>(p, mode, s);
+}

@@ -220,6 +220,9 @@ struct CrpParams {
 
 // launchers (return cudaGetLastError() after the launch)
 template <typename R> cudaError_t launch_column(const ColumnParams &p, int mode, cudaStream_t s);
+// FP64 column pass on the tensor cores; the bases it takes
+bool column_dmma_ok(int nth, int nl);
+cudaError_t launch_column_dmma(const ColumnParams &p, int mode, cudaStream_t s);
 template <typename R> cudaError_t launch_lines(const LineParams &p, cudaStream_t s);
 template <typename R> cudaError_t launch_flux_prep(const FluxParams &p, cudaStream_t s);
 cudaError_t launch_flux_accum(const AccumParams &p, cudaStream_t s);
