@@ -4,6 +4,7 @@
 //     expV[k][j][i] = exp(-i V dt)                       setup_exp_ipot_dt    timeEvol.C:438-463
 //     rot[l][j][i]  = exp(-i l(l+1)(I1_i + I2_j) dt/2)   setup_exp_irot_dt_2  timeEvol.C:465-491
 //     kin[j][i]     = exp(-i(T1_i + T2_j) dt) / n1 / n2  setup_exp_ikin_dt    timeEvol.C:493-517
+//   or, for the kernels of k_axis.cuh, the factors of rot and kin in R and in r
 //   FP32 form: exp(-i V dt) and the separable factors of the rotational and
 //   kinetic phases (exp(-i l(l+1) I1 dt/2), exp(-i l(l+1) I2 dt/2),
 //   exp(-i T1 dt), exp(-i T2 dt)), each evaluated in FP64 with the phase
@@ -26,9 +27,9 @@ __global__ void k_tables_fp64(int n1, int n2, int nth, int nl, double dt, const 
                               const double *T2, double2 *expV, double2 *rot, double2 *kin)
 {
   const long n12 = (long)n1 * n2;
-  const long nv = n12 * nth, nr = n12 * nl;
+  const long nv = n12 * nth, nr = rot ? n12 * nl : 0, nk = rot ? n12 : 0;
   const double mdt = -dt, mdt2 = -dt / 2;
-  for (long g = blockIdx.x * (long)blockDim.x + threadIdx.x; g < nv + nr + n12;
+  for (long g = blockIdx.x * (long)blockDim.x + threadIdx.x; g < nv + nr + nk;
        g += (long)gridDim.x * blockDim.x) {
     double s, c;
     if (g < nv) {
@@ -48,6 +49,39 @@ __global__ void k_tables_fp64(int n1, int n2, int nth, int nl, double dt, const 
       sincos((T1[i] + T2[j]) * mdt, &s, &c);
       kin[ij] = make_double2(c / n1 / n2, s / n1 / n2);
     }
+  }
+}
+
+// the separable factors of rot and kin (without the 1/(n1 n2))
+__global__ void k_factors_fp64(int n1, int n2, int nl, double dt, const double *I1,
+                               const double *I2, const double *T1, const double *T2, double2 *zr1,
+                               double2 *zr2, double2 *zk1, double2 *zk2)
+{
+  const int a1 = nl * n1, a2 = nl * n2;
+  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < a1 + a2 + n1 + n2;
+       g += gridDim.x * blockDim.x) {
+    double ph;
+    double2 *dst;
+    if (g < a1) {
+      const int l = g / n1;
+      ph = (double)(l * (l + 1)) * I1[g - l * n1] * (-dt / 2);
+      dst = zr1 + g;
+    } else if (g < a1 + a2) {
+      const int q = g - a1, l = q / n2;
+      ph = (double)(l * (l + 1)) * I2[q - l * n2] * (-dt / 2);
+      dst = zr2 + q;
+    } else if (g < a1 + a2 + n1) {
+      const int i = g - a1 - a2;
+      ph = T1[i] * -dt;
+      dst = zk1 + i;
+    } else {
+      const int j = g - a1 - a2 - n1;
+      ph = T2[j] * -dt;
+      dst = zk2 + j;
+    }
+    double s, c;
+    sincos(ph, &s, &c);
+    *dst = make_double2(c, s);
   }
 }
 
@@ -167,6 +201,16 @@ cudaError_t launch_setup_tables_fp64(int n1, int n2, int nth, int nl, double dt,
                                      double2 *rot, double2 *kin, cudaStream_t s)
 {
   k_tables_fp64<<<148 * 8, 256, 0, s>>>(n1, n2, nth, nl, dt, pot, I1, I2, T1, T2, expV, rot, kin);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_setup_factors_fp64(int n1, int n2, int nl, double dt, const double *I1,
+                                      const double *I2, const double *T1, const double *T2,
+                                      double2 *zr1, double2 *zr2, double2 *zk1, double2 *zk2,
+                                      cudaStream_t s)
+{
+  const int n = nl * (n1 + n2) + n1 + n2;
+  k_factors_fp64<<<(n + 255) / 256, 256, 0, s>>>(n1, n2, nl, dt, I1, I2, T1, T2, zr1, zr2, zk1, zk2);
   return cudaGetLastError();
 }
 

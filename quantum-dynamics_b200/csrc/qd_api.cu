@@ -561,6 +561,7 @@ struct qd_handle {
   double *d_I1 = nullptr, *d_I2 = nullptr, *d_T1 = nullptr, *d_T2 = nullptr;
   double *d_d1 = nullptr, *d_d2 = nullptr;
   double2 *d_expV = nullptr, *d_rot = nullptr, *d_kin = nullptr;
+  double2 *d_zr1 = nullptr, *d_zr2 = nullptr, *d_zk1 = nullptr, *d_zk2 = nullptr;
   float2 *d_expV32 = nullptr;
   float2 *d_rc1 = nullptr, *d_rc2 = nullptr, *d_kc1 = nullptr, *d_kc2 = nullptr;
   int slice_cluster = 0;          // l-space kernel (LineParams::cluster code)
@@ -829,7 +830,7 @@ template <typename R> int issue_column(qd_handle *h, int mode, bool flux, double
     // the surface rows of this step go to ring slot ring_fill; with the fused
     // slice kernel that preparation rides along in the next l-space launch
     h->flux_pending = h->ring_fill;
-    if (!(sizeof(R) == 4 && h->slice_cluster > 0 && !h->lines_split) || mode == COL_TAIL)
+    if (!(h->slice_cluster > 0 && !h->lines_split) || mode == COL_TAIL)
       TRY(issue_flux_prep<R>(h));
   }
   return QD_OK;
@@ -881,7 +882,8 @@ LineParams line_params(qd_handle *h, bool f32)
   p.nruns = h->nruns;
   p.rot = h->d_rot; p.kin = h->d_kin;
   p.rc1 = h->d_rc1; p.rc2 = h->d_rc2; p.kc1 = h->d_kc1; p.kc2 = h->d_kc2;
-  p.cluster = f32 ? h->slice_cluster : 0;
+  p.zr1 = h->d_zr1; p.zr2 = h->d_zr2; p.zk1 = h->d_zk1; p.zk2 = h->d_zk2;
+  p.cluster = h->slice_cluster;
   const double ks = 1.0 / ((double)h->n1 * h->n2);
   p.kscale = (float)ks;
   p.kscale_lo = (float)(ks - (double)p.kscale);
@@ -894,28 +896,67 @@ LineParams line_params(qd_handle *h, bool f32)
   return p;
 }
 
-// Autotuner of the complex64 l-space pass: time the fused slice kernel with
-// 1, 2 and 4 CTAs per slice, the register-FFT slice kernel on 1, 2 or 4
-// CTAs per slice (where built) and the split kernels on a scratch wavepacket and keep the
-// fastest; the choice is kept for later handles of the same shapes.
-// QD_SLICE_CLUSTER=0|1|2|4|8|9|10|11 forces a choice (8 = the register-FFT
-// kernel, 9 and 10 = the same on a 2- and a 4-CTA cluster).
+cudaError_t run_lines(const LineParams &p, bool f32, cudaStream_t st)
+{
+  if (f32) return p.cluster ? launch_slice(p, st) : launch_lines<float>(p, st);
+  return p.cluster ? launch_axis_f64(p, st) : launch_lines<double>(p, st);
+}
+
+// the FP64 l-space kernels beside the split ones: k_axis.cuh, where it takes
+// the grid (QD_SLICE_CLUSTER=0 keeps the split kernels)
+bool axis_f64(const qd_handle *h, bool fused)
+{
+  AxisPlan ax;
+  const char *force = getenv("QD_SLICE_CLUSTER");
+  return !(force && atoi(force) == 0) &&
+         axis_plan(h->n1, h->n2, sizeof(double2), fused, ax);
+}
+
+// Autotuner of the l-space pass: time the kernels that take the grid on the
+// handle's zero l-space buffer (a zero wavepacket stays zero) and keep the
+// fastest; the choice is kept for later handles of the same shapes.  The kernels that are tried, per grid:
+//   complex64, sizes compiled in: the register-FFT slice kernel on 1, 2 or 4
+//     CTAs per slice (128 x 96 x 64, one run: 14.8 us a step on two; run-time
+//     sizes 19.0, Stockham slice kernel 22.8);
+//   two built factors a side (k_axis.cuh): its fused form and its row and
+//     column launches, either of which may win (54 x 60 x 32 complex64: 15.8
+//     and 17.1 us; 144 x 120 x 64: 35 and 23 us; the Stockham kernels 25 and 51);
+//   other grids: the split kernels and (complex64) the Stockham slice kernel
+//     on 1, 2 and 4 CTAs per slice.
+// QD_SLICE_CLUSTER=0|1|2|4|8|9|10|11|12|13 forces a choice (0 the split
+// kernels, 1, 2, 4 the Stockham slice kernel, 8, 9, 10 the register-FFT kernel
+// on 1, 2 and 4 CTAs, 11 its wide form, 12, 13 the run-time one, fused or as two
+// launches; FP64 knows 0, 12 and 13 only).
 int tune_slice(qd_handle *h)
 {
   h->slice_cluster = 0;
-  if (h->prec != QD_PREC_FP32) return QD_OK;
+  const bool f32 = h->prec == QD_PREC_FP32;
+  auto built = [&](int cl) {
+    return f32 ? slice_cluster_ok(h->n1, h->n2, cl) != 0
+               : slice_is_ax(cl) && axis_f64(h, cl == SLICE_AX);
+  };
+  const bool rf = f32 && (built(SLICE_RF) || built(SLICE_RF2) || built(SLICE_RF4));
+  const bool ax = !rf && built(SLICE_AX2);
+  auto tried = [&](int cl) {
+    return rf ? slice_is_rf(cl) && built(cl) : ax ? slice_is_ax(cl) && built(cl)
+                                                 : cl == 0 || (!slice_is_ax(cl) && built(cl));
+  };
   const char *force = getenv("QD_SLICE_CLUSTER");
-  if (force) {
-    const int cl = atoi(force);
-    h->slice_cluster = slice_cluster_ok(h->n1, h->n2, cl) ? cl : 0;
-    return QD_OK;
+  const int forced = force ? atoi(force) : 0;
+  if (force && (f32 || forced == 0 || slice_is_ax(forced))) {
+    if (forced) h->slice_cluster = built(forced) ? forced : 0;
+    if (f32 || forced == 0 || h->slice_cluster) return QD_OK;
+  }
+  if (!f32) {
+    if (!ax) return QD_OK;
+    h->slice_cluster = SLICE_AX2;       // the tables of the split kernels are not built
   }
   // the choice depends on the shapes only: measured once per process and device
   static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int, int, int, int>, int> chosen;
+  static std::map<std::tuple<int, int, int, int, int, int, int, int>, int> chosen;
   int dev = 0;
   cudaGetDevice(&dev);
-  const auto key = std::make_tuple(dev, h->n1, h->n2, h->nl, h->nruns, h->jrows,
+  const auto key = std::make_tuple(dev, h->prec, h->n1, h->n2, h->nl, h->nruns, h->jrows,
                                    h->d_run_k ? 1 : 0);
   {
     std::lock_guard<std::mutex> lock(mu);
@@ -925,25 +966,20 @@ int tune_slice(qd_handle *h)
       return QD_OK;
     }
   }
-  void *scratch = nullptr;
-  const size_t sbytes = sizeof(float2) * h->n12 * h->nl * h->nruns;
-  CU(cudaMallocAsync(&scratch, sbytes, h->st));
-  CU(cudaMemsetAsync(scratch, 0, sbytes, h->st));
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
-  LineParams p = line_params(h, true);
-  p.lpsi = scratch;
+  LineParams p = line_params(h, f32);
   float best = 1e30f;
-  for (int cl : {0, 1, 2, 4, SLICE_RF, SLICE_RF2, SLICE_RF4, SLICE_RF4W}) {
-    if (cl > 0 && !slice_cluster_ok(h->n1, h->n2, cl)) continue;
+  for (int cl : {0, 1, 2, 4, SLICE_RF, SLICE_RF2, SLICE_RF4, SLICE_RF4W, SLICE_AX, SLICE_AX2}) {
+    if (!tried(cl)) continue;
     p.cluster = cl;
     bool ok = true;
     for (int it = 0; it < 2 && ok; it++)
-      ok = (cl ? launch_slice(p, h->st) : launch_lines<float>(p, h->st)) == cudaSuccess;
+      ok = run_lines(p, f32, h->st) == cudaSuccess;
     if (ok) ok = cudaEventRecord(e0, h->st) == cudaSuccess;
     for (int it = 0; it < 5 && ok; it++)
-      ok = (cl ? launch_slice(p, h->st) : launch_lines<float>(p, h->st)) == cudaSuccess;
+      ok = run_lines(p, f32, h->st) == cudaSuccess;
     if (ok) ok = cudaEventRecord(e1, h->st) == cudaSuccess;
     if (ok) ok = cudaStreamSynchronize(h->st) == cudaSuccess;
     float ms = 0.f;
@@ -956,7 +992,8 @@ int tune_slice(qd_handle *h)
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  CU(cudaFreeAsync(scratch, h->st));
+  CU(cudaMemsetAsync(h->d_lpsi, 0, (f32 ? sizeof(float2) : sizeof(double2)) * h->n12 * h->nl *
+                                       h->nruns, h->st));
   std::lock_guard<std::mutex> lock(mu);
   chosen[key] = h->slice_cluster;
   return QD_OK;
@@ -1075,13 +1112,9 @@ template <typename R> int issue_lines(qd_handle *h)
     p.flux_ctas = (ctas + cl - 1) / cl * cl;
   }
   TRY(prof_mark(h, -1));
-  if (p.cluster > 0) {
-    CU(launch_slice(p, h->st));
-    g_launches++;
-  } else {
-    CU(launch_lines<R>(p, h->st));
-    g_launches += lines_launches_per_step(h->n1, h->n2, h->prec);
-  }
+  CU(run_lines(p, sizeof(R) == 4, h->st));
+  g_launches += p.cluster == 0 ? lines_launches_per_step(h->n1, h->n2, h->prec)
+              : p.cluster == SLICE_AX2 ? 2 : 1;
   TRY(prof_mark(h, PROF_LINES));
   if (fused_flux) TRY(after_flux_prep(h));
   return QD_OK;
@@ -1181,8 +1214,8 @@ template <typename Real> int propagate(qd_handle *h, int n, size_t flush_bytes =
     if (every <= 0 || t <= steps0 || t > steps0 + n || t % every) return nullptr;
     return h->d_esum + (long)(t / every - steps0 / every - 1) * R * 3;
   };
-  const bool split_ok = h->prec == QD_PREC_FP64 || h->slice_cluster == 0 ||
-                        slice_is_rf(h->slice_cluster);
+  const bool split_ok = h->slice_cluster == 0 || slice_is_rf(h->slice_cluster) ||
+                        slice_is_ax(h->slice_cluster);
   for (int s = 0; s < n; s++) {
     const bool redo = !h->started || (s == 0 && h->last_finalized);
     h->esum_col = redo ? nullptr : slot(h->steps);
@@ -1467,8 +1500,18 @@ int create(const qd_data *runs, int nruns, qd_handle **out)
   }
   if (f64) {
     TRY(h->alloc(h->d_expV, npt * npot));
-    TRY(h->alloc(h->d_rot, (size_t)h->n12 * h->jrows));
-    TRY(h->alloc(h->d_kin, h->n12));
+    if (axis_f64(h, false)) {
+      TRY(h->alloc(h->d_zr1, (size_t)h->jrows * h->n1));
+      TRY(h->alloc(h->d_zr2, (size_t)h->jrows * h->n2));
+      TRY(h->alloc(h->d_zk1, h->n1));
+      TRY(h->alloc(h->d_zk2, h->n2));
+      CU(launch_setup_factors_fp64(h->n1, h->n2, h->jrows, h->dt, h->d_I1, h->d_I2, h->d_T1,
+                                   h->d_T2, h->d_zr1, h->d_zr2, h->d_zk1, h->d_zk2, h->st));
+      g_launches++;
+    } else {
+      TRY(h->alloc(h->d_rot, (size_t)h->n12 * h->jrows));
+      TRY(h->alloc(h->d_kin, h->n12));
+    }
     CU(launch_setup_tables_fp64(h->n1, h->n2, h->nth * npot, h->jrows, h->dt, h->d_pot, h->d_I1,
                                 h->d_I2, h->d_T1, h->d_T2, h->d_expV, h->d_rot, h->d_kin,
                                 h->st));
@@ -1947,7 +1990,7 @@ int qd_set_profiling(qd_handle *h, int32_t on)
 int qd_kernel_choice(qd_handle *h, int32_t out[4])
 {
   if (!h || !out) return set_err(QD_ERR_INVALID, "NULL argument");
-  out[0] = h->slice_cluster;
+  out[0] = h->prec == QD_PREC_FP32 ? h->slice_cluster : 0;
   out[1] = h->use_tc ? 1 : 0;
   out[2] = h->flux_variant;
   out[3] = h->d_czt_b ? 1 : 0;
