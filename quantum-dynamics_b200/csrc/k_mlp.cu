@@ -9,16 +9,17 @@
 //   p_ij = exp(-r_ij / 1.5 bohr),  f = (p23, p12 + p13, p12 p13),
 // invariant under exchanging atoms 2 and 3, standardised; then four dense
 // layers of width 64 with SiLU, and a linear scalar output (standardised V).
-// Weights: FP32 master copies for Adam, and an FP32 copy (wq) that every
-// forward and backward product reads, FP32 accumulation.  (Products on
-// BF16-rounded weights left 5.3 meV RMS on the C1 grid against 3.0 meV with
-// FP32 weights, same training.)
+// Weights, products, accumulation and Adam are FP32.  (Products on BF16-rounded
+// weights left 5.3 meV RMS on the C1 grid against 3.0 meV with FP32 weights,
+// same training.)
 //
-// Training kernels over a minibatch of n samples (activations [n][64] in
-// global memory, L2-resident): dense forward (Z = A W^T + b, A' = SiLU(Z)),
-// output layer and loss, backward through the output, backward data
-// (D_prev = (D W) * SiLU'(Z_prev)), weight gradients (G = D^T A_prev, summed
-// over the batch in registers per CTA, then one atomic add per entry), Adam.
+// A training step is two launches.  k_mlp_step takes tiles of 32 samples
+// through the whole network in shared memory, forward and backward, with all
+// weights beside them; the weight gradients of a CTA's tiles stay in registers
+// (49 per thread) and go out once, as that CTA's row of a partial array.
+// k_mlp_adam sums the rows in order and updates the weights.  (One launch per
+// layer and direction, activations in global memory and the weight gradients
+// on 8 CTAs with atomics, took 342 us a step at 4096 samples; this form takes 22.)
 // Inference: one fused kernel per tile of 64 points (features from the
 // Jacobi geometry, all layers in shared memory).
 #include <cmath>
@@ -68,208 +69,325 @@ __global__ void k_features(int n, const double *r12, const double *r23, const do
   }
 }
 
-// Z[s][o] = sum_k A[s][k] Wt[o][k] + b[o], A'[s][o] = SiLU(Z).  CTA: 64 samples x
-// 64 outputs, 256 threads with 4 x 4 outputs each (rows tr + 16 i, cols tc + 16 j).
-__global__ void __launch_bounds__(256) k_dense_fwd(int n, int K, const float *A, const float *Wt,
-                                                   const float *b, float *Z, float *Aout)
-{
-  __shared__ float As[64][W + 1], Ws[W][W + 1];
-  const int tid = threadIdx.x, tr = tid >> 4, tc = tid & 15, s0 = blockIdx.x * 64;
-  for (int x = tid; x < 64 * K; x += 256) {
-    const int r = x / K, k = x % K;
-    As[r][k] = s0 + r < n ? A[(long)(s0 + r) * K + k] : 0.f;
-    Ws[r][k] = Wt[r * K + k];
-  }
-  __syncthreads();
-  float acc[4][4];
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = b[tc + 16 * j];
-  for (int k = 0; k < K; k++) {
-    float a[4], w[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) a[i] = As[tr + 16 * i][k];
-#pragma unroll
-    for (int j = 0; j < 4; j++) w[j] = Ws[tc + 16 * j][k];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int s = s0 + tr + 16 * i;
-    if (s >= n) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      Z[(long)s * W + tc + 16 * j] = acc[i][j];
-      Aout[(long)s * W + tc + 16 * j] = silu(acc[i][j]);
-    }
-  }
-}
+// Forward and backward over samples [0, n) in tiles of TS, one CTA to a tile at
+// a time: part[blockIdx][0..NPARAM) = this CTA's share of d(mean squared
+// error)/d(parameters) (GRADS), part[blockIdx][NPARAM] its sum of squared errors.
+// 256 threads; a layer's 32 x 64 outputs are 2 samples x 4 outputs a thread with
+// the contraction read four at a time (6 16-byte loads per 32 FMAs), its weight
+// gradient 4 x 4 entries a thread over the 32 samples (2 per 16).
+// Bound: the latency of the chain of layers at two warps per scheduler (one
+// tile of a 4096-sample batch per CTA: 9200 FMAs per scheduler, 4 us at the FMA
+// rate, in about 16 us); smaller tiles would not fill more SMs by much and
+// double the weight traffic per sample.
+constexpr int TS = 32;                    // samples of a tile
+constexpr int LDA = W + 4;                // row stride: 16-byte rows, conflict-free quarter-warps
+constexpr int PSTRIDE = (NPARAM + 1 + 3) / 4 * 4;
+struct StepSmem {
+  float w[NL - 1][W][LDA];                // layers 2..4
+  float a[NL][TS][LDA], s[NL][TS][LDA];   // activations, SiLU'(z)
+  float d[2][TS][LDA];                    // backward signal, ping-pong
+  float f[TS][4];                         // features, and 1 for the bias
+  float e[TS];                            // 2 (y - t) / n_total
+  float w1[W][NF], b[NL][W], wo[W];
+};
 
-// output layer, loss and its gradient: y = A4 . wo + bo, e = 2 (y - t) / n_total,
-// D4[s][k] = e wo[k] SiLU'(Z4[s][k]); the loss sum goes to *loss
-__global__ void __launch_bounds__(256) k_out_loss(int n, float inv_total, const float *A4,
-                                                  const float *Z4, const float *wo, const float *bo,
-                                                  const float *target, float *y, float *D4,
-                                                  float *loss)
+template <bool GRADS>
+__global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, const float *F,
+                                                     const float *target, const float *w,
+                                                     float *part)
 {
+  extern __shared__ float4 step_sm4[];
+  StepSmem &m = *reinterpret_cast<StepSmem *>(step_sm4);
   __shared__ float red[8];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int s = blockIdx.x * 8 + warp;            // one warp per sample
-  float l2 = 0.f;
-  if (s < n) {
-    float acc = A4[(long)s * W + lane] * wo[lane] + A4[(long)s * W + lane + 32] * wo[lane + 32];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    const float yp = acc + bo[0];
-    const float d = yp - (target ? target[s] : 0.f);
-    if (lane == 0) {
-      if (y) y[s] = yp;
-      l2 = d * d;
-    }
-    if (D4) {
-      const float e = 2.f * d * inv_total;
-      D4[(long)s * W + lane] = e * wo[lane] * dsilu(Z4[(long)s * W + lane]);
-      D4[(long)s * W + lane + 32] = e * wo[lane + 32] * dsilu(Z4[(long)s * W + lane + 32]);
-    }
-  }
-  if (lane == 0) red[warp] = l2;
-  __syncthreads();
-  if (threadIdx.x == 0 && loss) {
-    float t = 0.f;
-    for (int w = 0; w < 8; w++) t += red[w];
-    atomicAdd(loss, t);
-  }
-}
-
-// Dp[s][k] = (sum_o D[s][o] Wt[o][k]) * SiLU'(Zp[s][k]) for the layer below (K = 64)
-__global__ void __launch_bounds__(256) k_dense_bwd_data(int n, const float *D, const float *Wt,
-                                                        const float *Zp, float *Dp)
-{
-  __shared__ float Ds[64][W + 1], Ws[W][W + 1];
-  const int tid = threadIdx.x, tr = tid >> 4, tc = tid & 15, s0 = blockIdx.x * 64;
-  for (int x = tid; x < 64 * W; x += 256) {
-    const int r = x / W, k = x % W;
-    Ds[r][k] = s0 + r < n ? D[(long)(s0 + r) * W + k] : 0.f;
-    Ws[r][k] = Wt[r * W + k];
-  }
-  __syncthreads();
-  float acc[4][4] = {};
-  for (int o = 0; o < W; o++) {
-    float d[4], w[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) d[i] = Ds[tr + 16 * i][o];
-#pragma unroll
-    for (int j = 0; j < 4; j++) w[j] = Ws[o][tc + 16 * j];
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-#pragma unroll
-      for (int j = 0; j < 4; j++) acc[i][j] = fmaf(d[i], w[j], acc[i][j]);
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int s = s0 + tr + 16 * i;
-    if (s >= n) continue;
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const long q = (long)s * W + tc + 16 * j;
-      Dp[q] = acc[i][j] * dsilu(Zp[q]);
-    }
-  }
-}
-
-// G[o][k] += sum_s D[s][o] Ap[s][k], gb[o] += sum_s D[s][o] over this CTA's
-// chunk of samples (K <= 64; Ap = features for the first layer, then A)
-constexpr int GCHUNK = 512;
-__global__ void __launch_bounds__(256) k_dense_bwd_weight(int n, int K, const float *D,
-                                                          const float *Ap, float *G, float *gb)
-{
-  __shared__ float Ds[64][W + 1], As[64][W + 1];
   const int tid = threadIdx.x, tr = tid >> 4, tc = tid & 15;
-  float acc[4][4] = {};
-  float accb[4] = {};
-  const int sb = blockIdx.x * GCHUNK, se = min(n, sb + GCHUNK);
-  for (int s0 = sb; s0 < se; s0 += 64) {
-    for (int x = tid; x < 64 * W; x += 256) {
-      const int r = x / W, c = x % W;
-      const bool ok = s0 + r < se;
-      Ds[r][c] = ok ? D[(long)(s0 + r) * W + c] : 0.f;
-      As[r][c] = (ok && c < K) ? Ap[(long)(s0 + r) * K + c] : 0.f;
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");     // the weights: the last step's update
+  {                                       // 16-byte weight rows, all loads in flight together
+    constexpr int PT = W * W / 4 / 256;
+    float4 v[NL - 1][PT];
+#pragma unroll
+    for (int l = 1; l < NL; l++)
+#pragma unroll
+      for (int q = 0; q < PT; q++)
+        v[l - 1][q] = reinterpret_cast<const float4 *>(w + layer_off(l))[tid + 256 * q];
+#pragma unroll
+    for (int l = 1; l < NL; l++)
+#pragma unroll
+      for (int q = 0; q < PT; q++) {
+        const int x = tid + 256 * q;
+        *reinterpret_cast<float4 *>(&m.w[l - 1][x / (W / 4)][4 * (x % (W / 4))]) = v[l - 1][q];
+      }
+  }
+  for (int x = tid; x < W * NF; x += 256) m.w1[x / NF][x % NF] = w[x];
+  for (int x = tid; x < NL * W; x += 256)
+    m.b[x / W][x % W] = w[layer_off(x / W) + W * (x / W ? W : NF) + x % W];
+  if (tid < W) m.wo[tid] = w[OFF_WO + tid];
+  const float bo = w[OFF_BO];
+  static_assert(layer_off(1) % 4 == 0 && (W * W + W) % 4 == 0, "16-byte weight rows");
+
+  float g[NL - 1][4][4] = {};             // dW of layers 2..4, entries [4 tr + i][4 tc + j]
+  float g1 = 0.f;                         // layer 1: dW[tid / 4][tid % 4], the bias at 3
+  float gb[NL - 1] = {};                  // biases of layers 2..4 (tid < 64)
+  float go = 0.f, gbo = 0.f;              // output weight tid - 64 and its bias
+  float l2 = 0.f;
+  for (int s0 = blockIdx.x * TS; s0 < n; s0 += gridDim.x * TS) {
+    if (tid < TS) {
+      const bool ok = s0 + tid < n;
+      const float *f = F + (long)(s0 + tid) * NF;
+#pragma unroll
+      for (int c = 0; c < NF; c++) m.f[tid][c] = ok ? f[c] : 0.f;
+      m.f[tid][3] = 1.f;
     }
-    __syncthreads();
-    for (int r = 0; r < 64; r++) {
-      float d[4], a[4];
+    __syncthreads();                      // features (and, first time, the weights) in place
+    {                                     // layer 1: output o of samples s
+      const int o = tid & (W - 1);
+      const float w0 = m.w1[o][0], w1 = m.w1[o][1], w2 = m.w1[o][2], b = m.b[0][o];
 #pragma unroll
-      for (int i = 0; i < 4; i++) d[i] = Ds[r][tr + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; j++) a[j] = As[r][tc + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        if (tc == 0) accb[i] += d[i];
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(d[i], a[j], acc[i][j]);
+      for (int s = tid / W; s < TS; s += 256 / W) {
+        const float z = fmaf(m.f[s][2], w2, fmaf(m.f[s][1], w1, fmaf(m.f[s][0], w0, b)));
+        m.a[0][s][o] = silu(z);
+        if (GRADS) m.s[0][s][o] = dsilu(z);
       }
     }
     __syncthreads();
+#pragma unroll 1
+    for (int l = 1; l < NL; l++) {
+      float acc[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = m.b[l][tc + 16 * j];
+#pragma unroll
+      for (int k = 0; k < W; k += 4) {
+        float4 a[2], v[4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) a[i] = *reinterpret_cast<const float4 *>(&m.a[l - 1][tr + 16 * i][k]);
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[j] = *reinterpret_cast<const float4 *>(&m.w[l - 1][tc + 16 * j][k]);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+            acc[i][j] = fmaf(a[i].w, v[j].w, fmaf(a[i].z, v[j].z,
+                        fmaf(a[i].y, v[j].y, fmaf(a[i].x, v[j].x, acc[i][j]))));
+      }
+#pragma unroll
+      for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          m.a[l][tr + 16 * i][tc + 16 * j] = silu(acc[i][j]);
+          if (GRADS) m.s[l][tr + 16 * i][tc + 16 * j] = dsilu(acc[i][j]);
+        }
+      __syncthreads();
+    }
+    {                                     // output, loss and its gradient: 8 threads a sample
+      const int s = tid >> 3, k0 = (tid & 7) * 4;
+      float acc = 0.f;
+#pragma unroll
+      for (int k = k0; k < W; k += 32)
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc = fmaf(m.a[NL - 1][s][k + i], m.wo[k + i], acc);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      const float d = s0 + s < n ? acc + bo - target[s0 + s] : 0.f;
+      const float e = 2.f * d * inv_total;
+      if ((tid & 7) == 0) {
+        l2 = fmaf(d, d, l2);
+        m.e[s] = e;
+      }
+      if (GRADS)
+#pragma unroll
+        for (int k = k0; k < W; k += 32)
+#pragma unroll
+          for (int i = 0; i < 4; i++) m.d[0][s][k + i] = e * m.wo[k + i] * m.s[NL - 1][s][k + i];
+    }
+    __syncthreads();
+    if (!GRADS) continue;
+    if (tid >= W && tid < 2 * W)          // output weights
+#pragma unroll 8
+      for (int s = 0; s < TS; s++) {
+        go = fmaf(m.e[s], m.a[NL - 1][s][tid - W], go);
+        gbo += m.e[s];
+      }
+#pragma unroll
+    for (int l = NL - 1; l >= 1; l--) {
+      float (*D)[LDA] = m.d[(NL - 1 - l) & 1], (*Dp)[LDA] = m.d[(NL - l) & 1];
+      // dW[o][k] = sum_s D[s][o] A[s][k]
+#pragma unroll 16
+      for (int s = 0; s < TS; s++) {
+        const float4 x = *reinterpret_cast<const float4 *>(&D[s][4 * tr]);
+        const float4 y = *reinterpret_cast<const float4 *>(&m.a[l - 1][s][4 * tc]);
+        const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int j = 0; j < 4; j++) g[l - 1][i][j] = fmaf(xs[i], ys[j], g[l - 1][i][j]);
+      }
+      if (tid < W)
+#pragma unroll 8
+        for (int s = 0; s < TS; s++) gb[l - 1] += D[s][tid];
+      // D below: (sum_o D[s][o] W[o][k]) SiLU'(z[s][k]), samples tr, tr + 16, k = 4 tc + j
+      float acc[2][4] = {};
+#pragma unroll
+      for (int o = 0; o < W; o += 4) {
+        float4 x[2], v[4];
+#pragma unroll
+        for (int i = 0; i < 2; i++) x[i] = *reinterpret_cast<const float4 *>(&D[tr + 16 * i][o]);
+#pragma unroll
+        for (int q = 0; q < 4; q++) v[q] = *reinterpret_cast<const float4 *>(&m.w[l - 1][o + q][4 * tc]);
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          const float xs[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            acc[i][0] = fmaf(xs[q], v[q].x, acc[i][0]);
+            acc[i][1] = fmaf(xs[q], v[q].y, acc[i][1]);
+            acc[i][2] = fmaf(xs[q], v[q].z, acc[i][2]);
+            acc[i][3] = fmaf(xs[q], v[q].w, acc[i][3]);
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int s = tr + 16 * i;
+        const float4 z = *reinterpret_cast<const float4 *>(&m.s[l - 1][s][4 * tc]);
+        *reinterpret_cast<float4 *>(&Dp[s][4 * tc]) =
+            make_float4(acc[i][0] * z.x, acc[i][1] * z.y, acc[i][2] * z.z, acc[i][3] * z.w);
+      }
+      __syncthreads();
+    }
+#pragma unroll 8
+    for (int s = 0; s < TS; s++) g1 = fmaf(m.d[(NL - 1) & 1][s][tid >> 2], m.f[s][tid & 3], g1);
+    __syncthreads();                      // before the next tile's features
   }
+
+  float *out = part + (size_t)blockIdx.x * PSTRIDE;
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int o = tr + 16 * i;
-    if (tc == 0) atomicAdd(gb + o, accb[i]);
+  for (int o = 16; o > 0; o >>= 1) l2 += __shfl_xor_sync(0xffffffffu, l2, o);
+  if ((tid & 31) == 0) red[tid >> 5] = l2;
+  __syncthreads();
+  if (tid == 0) {
+    float t = 0.f;
+    for (int x = 0; x < 8; x++) t += red[x];
+    out[NPARAM] = t;
+  }
+  if (!GRADS) return;
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int k = tc + 16 * j;
-      if (k < K) atomicAdd(G + o * K + k, acc[i][j]);
+  for (int l = 1; l < NL; l++) {
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+      *reinterpret_cast<float4 *>(out + layer_off(l) + (4 * tr + i) * W + 4 * tc) =
+          make_float4(g[l - 1][i][0], g[l - 1][i][1], g[l - 1][i][2], g[l - 1][i][3]);
+    if (tid < W) out[layer_off(l) + W * W + tid] = gb[l - 1];
+  }
+  if ((tid & 3) < NF) out[(tid >> 2) * NF + (tid & 3)] = g1;
+  else out[W * NF + (tid >> 2)] = g1;
+  if (tid >= W && tid < 2 * W) out[OFF_WO + tid - W] = go;
+  if (tid == W) out[OFF_BO] = gbo;
+}
+
+// Sums the partial rows of a step: the gradient of parameter p into grad (if
+// given, no update), else Adam; the squared errors are added to *loss (set if
+// `first`).  32 parameters a CTA, eight threads each over the rows in turn.
+struct AdamArgs { float lr, b1, b2, eps, c1, c2; };
+__global__ void __launch_bounds__(256) k_mlp_adam(int rows, const float *part, float *w, float *m,
+                                                  float *v, AdamArgs a, int first, float *loss,
+                                                  float *grad)
+{
+  __shared__ float red[8][33];
+  const int q = threadIdx.x & 31, r0 = threadIdx.x >> 5, p = blockIdx.x * 32 + q;
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");     // the step's partial rows
+  float t = 0.f;
+  if (p <= NPARAM)
+#pragma unroll 16
+    for (int r = r0; r < rows; r += 8) t += part[(size_t)r * PSTRIDE + p];
+  red[r0][q] = t;
+  __syncthreads();
+  if (r0 != 0 || p > NPARAM) return;
+  float g = 0.f;
+#pragma unroll
+  for (int x = 0; x < 8; x++) g += red[x][q];
+  if (p == NPARAM) {
+    *loss = first ? g : *loss + g;
+  } else if (grad) {
+    grad[p] = g;
+  } else {
+    const float mi = a.b1 * m[p] + (1.f - a.b1) * g, vi = a.b2 * v[p] + (1.f - a.b2) * g * g;
+    m[p] = mi;
+    v[p] = vi;
+    w[p] -= a.lr * (mi / a.c1) / (sqrtf(vi / a.c2) + a.eps);
+  }
+}
+
+// sums of the unstandardised features and V and of their squares, eight per CTA
+__global__ void __launch_bounds__(256) k_mlp_moments(long n, const double *r12, const double *r23,
+                                                     const double *r13, const double *V, double *out)
+{
+  __shared__ double red[8][8];
+  double s[8] = {};
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    const double p12 = exp(-r12[i] / FEAT_SCALE), p23 = exp(-r23[i] / FEAT_SCALE),
+                 p13 = exp(-r13[i] / FEAT_SCALE);
+    const double f[4] = {p23, p12 + p13, p12 * p13, V[i]};
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+      s[c] += f[c];
+      s[4 + c] += f[c] * f[c];
     }
   }
-}
-
-// output-layer gradients: gwo[k] = sum_s e_s A4[s][k] with e_s = D4 / (wo SiLU')
-// recomputed from y and the targets; done as G = E^T A4 with E the scalar errors
-__global__ void __launch_bounds__(256) k_out_grad(int n, float inv_total, const float *A4,
-                                                  const float *y, const float *target, float *gwo,
-                                                  float *gbo)
-{
-  __shared__ float red[W][9];
-  const int k = threadIdx.x & 63, part = threadIdx.x >> 6;   // 4 parts of the chunk
-  float acc = 0.f, accb = 0.f;
-  const int sb = blockIdx.x * GCHUNK, se = min(n, sb + GCHUNK);
-  for (int s = sb + part; s < se; s += 4) {
-    const float e = 2.f * (y[s] - target[s]) * inv_total;
-    acc = fmaf(e, A4[(long)s * W + k], acc);
-    if (k == 0) accb += e;
+#pragma unroll
+  for (int c = 0; c < 8; c++) {
+    for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5][c] = s[c];
   }
-  red[k][part] = acc;
-  red[k][4 + part] = accb;
   __syncthreads();
-  if (threadIdx.x < W) {
-    const float t = red[k][0] + red[k][1] + red[k][2] + red[k][3];
-    atomicAdd(gwo + k, t);
-    if (k == 0) atomicAdd(gbo, red[0][4] + red[0][5] + red[0][6] + red[0][7]);
+  if (threadIdx.x < 8) {
+    double t = 0.0;
+    for (int x = 0; x < 8; x++) t += red[x][threadIdx.x];
+    out[blockIdx.x * 8 + threadIdx.x] = t;
   }
 }
 
-// Adam on the FP32 masters; their copies feed the products
-__global__ void k_adam(int np, float *w, float *wq, const float *g, float *m, float *v, float lr,
-                       float b1, float b2, float eps, float c1, float c2)
+// standardised targets
+__global__ void k_targets(long n, const double *V, Norm nm, float *T)
 {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x) {
-    const float gi = g[i];
-    const float mi = b1 * m[i] + (1.f - b1) * gi, vi = b2 * v[i] + (1.f - b2) * gi * gi;
-    m[i] = mi;
-    v[i] = vi;
-    const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-    w[i] = wi;
-    wq[i] = wi;
-  }
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    T[i] = (float)((V[i] - nm.vmean) / nm.vstd);
 }
 
-__global__ void k_copy_weights(int np, const float *w, float *wq)
+// a launch that lets the next kernel's prologue overlap it (both kernels of a
+// step wait for the one before at entry)
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*k)(P...), unsigned grid, size_t smem, A... args)
 {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < np; i += gridDim.x * blockDim.x)
-    wq[i] = w[i];
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(256);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  qd_count_launches(1);
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+template <bool GRADS>
+cudaError_t launch_step(int rows, int n, float inv_total, const float *F, const float *T,
+                        const float *w, float *part)
+{
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_mlp_step<GRADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(StepSmem));
+  if (e != cudaSuccess) return e;
+  return launch_chained(k_mlp_step<GRADS>, (unsigned)rows, sizeof(StepSmem), n, inv_total, F, T, w, part);
+}
+
+cudaError_t launch_adam(int rows, const float *part, float *w, float *m, float *v, const AdamArgs &a,
+                        int first, float *loss, float *grad)
+{
+  return launch_chained(k_mlp_adam, (NPARAM + 32) / 32, 0, rows, part, w, m, v, a, first, loss, grad);
 }
 
 // Fused inference on the Jacobi grid (H3/H3PESJacobi.m:5-27 geometry): per
@@ -391,11 +509,11 @@ cudaError_t launch_mlp_grid(long blocks, const GridArgs &g, const Norm &nm, cons
 struct qd_mlp {
   Norm norm{};
   std::vector<float> w;                 // FP32 masters (host copy)
-  float *d_w = nullptr, *d_wq = nullptr, *d_m = nullptr, *d_v = nullptr, *d_g = nullptr;
+  float *d_w = nullptr, *d_m = nullptr, *d_v = nullptr;
   long step = 0;
   ~qd_mlp()
   {
-    for (float *p : {d_w, d_wq, d_m, d_v, d_g}) cudaFree(p);
+    for (float *p : {d_w, d_m, d_v}) cudaFree(p);
   }
 };
 
@@ -410,21 +528,9 @@ uint64_t mix(uint64_t &s)
   return z ^ (z >> 31);
 }
 
-void host_features(double r12, double r23, double r13, double *f)
-{
-  const double p12 = std::exp(-r12 / FEAT_SCALE), p23 = std::exp(-r23 / FEAT_SCALE),
-               p13 = std::exp(-r13 / FEAT_SCALE);
-  f[0] = p23;
-  f[1] = p12 + p13;
-  f[2] = p12 * p13;
-}
-
 int upload_params(qd_mlp *m)
 {
   QD_CU(cudaMemcpy(m->d_w, m->w.data(), sizeof(float) * NPARAM, cudaMemcpyHostToDevice));
-  k_copy_weights<<<(NPARAM + 255) / 256, 256>>>(NPARAM, m->d_w, m->d_wq);
-  qd_count_launches(1);
-  QD_CU(cudaGetLastError());
   return QD_OK;
 }
 
@@ -448,7 +554,7 @@ int qd_mlp_create(qd_mlp **out, uint64_t seed)
   for (int c = 0; c < NF; c++) { m->norm.fmean[c] = 0.f; m->norm.fstd[c] = 1.f; }
   m->norm.vmean = 0.f;
   m->norm.vstd = 1.f;
-  for (float **p : {&m->d_w, &m->d_wq, &m->d_m, &m->d_v, &m->d_g})
+  for (float **p : {&m->d_w, &m->d_m, &m->d_v})
     if (cudaMalloc(p, sizeof(float) * NPARAM) != cudaSuccess) {
       cudaGetLastError();
       delete m;
@@ -494,27 +600,34 @@ int qd_mlp_set_params(qd_mlp *m, const float *w, const float norm[8])
   return upload_params(m);
 }
 
-// standardisation of features and targets from a training set (host, FP64)
+// standardisation of features and targets from a training set: FP64 sums on the
+// device, one row per CTA, added up here in order
 int qd_mlp_fit_normalisation(qd_mlp *m, int64_t n, const double *r12, const double *r23,
                              const double *r13, const double *V)
 {
   if (!m || n < 2 || !r12 || !r23 || !r13 || !V) return qd_errf(QD_ERR_INVALID, "bad argument");
-  double s[NF] = {}, s2[NF] = {}, sv = 0.0, sv2 = 0.0;
-  for (int64_t i = 0; i < n; i++) {
-    double f[NF];
-    host_features(r12[i], r23[i], r13[i], f);
-    for (int c = 0; c < NF; c++) { s[c] += f[c]; s2[c] += f[c] * f[c]; }
-    sv += V[i];
-    sv2 += V[i] * V[i];
+  const int blocks = (int)((n + 255) / 256 < 148 * 4 ? (n + 255) / 256 : 148 * 4);
+  qd_scratch buf(sizeof(double) * (4 * (size_t)n + 8 * blocks));
+  double *d = buf.at<double>();
+  if (!d) return qd_errf(QD_ERR_NOMEM, "qd_mlp_fit_normalisation: %zu bytes", buf.bytes);
+  const double *src[4] = {r12, r23, r13, V};
+  for (int q = 0; q < 4; q++)
+    QD_CU(cudaMemcpy(d + q * n, src[q], sizeof(double) * n, cudaMemcpyHostToDevice));
+  k_mlp_moments<<<blocks, 256>>>(n, d, d + n, d + 2 * n, d + 3 * n, d + 4 * n);
+  qd_count_launches(1);
+  QD_CU(cudaGetLastError());
+  std::vector<double> rows(8 * (size_t)blocks);
+  QD_CU(cudaMemcpy(rows.data(), d + 4 * n, sizeof(double) * rows.size(), cudaMemcpyDeviceToHost));
+  double s[8] = {};
+  for (int b = 0; b < blocks; b++)
+    for (int c = 0; c < 8; c++) s[c] += rows[8 * b + c];
+  float *mean[4] = {&m->norm.fmean[0], &m->norm.fmean[1], &m->norm.fmean[2], &m->norm.vmean};
+  float *std[4] = {&m->norm.fstd[0], &m->norm.fstd[1], &m->norm.fstd[2], &m->norm.vstd};
+  for (int c = 0; c < 4; c++) {
+    const double mu = s[c] / n, var = s[4 + c] / n - mu * mu;
+    *mean[c] = (float)mu;
+    *std[c] = (float)std::sqrt(var > 1e-30 ? var : 1e-30);
   }
-  for (int c = 0; c < NF; c++) {
-    const double mu = s[c] / n, var = s2[c] / n - mu * mu;
-    m->norm.fmean[c] = (float)mu;
-    m->norm.fstd[c] = (float)std::sqrt(var > 1e-30 ? var : 1e-30);
-  }
-  const double mu = sv / n, var = sv2 / n - mu * mu;
-  m->norm.vmean = (float)mu;
-  m->norm.vstd = (float)std::sqrt(var > 1e-30 ? var : 1e-30);
   return QD_OK;
 }
 
@@ -530,116 +643,58 @@ int qd_mlp_train(qd_mlp *m, int64_t n, const double *r12, const double *r23, con
   if (!m || n < 1 || !r12 || !r23 || !r13 || !V || batch < 1)
     return qd_errf(QD_ERR_INVALID, "qd_mlp_train: bad argument");
   const int B = (int)(train_steps > 0 ? (batch < n ? batch : n) : n);
-  // device data: features and standardised targets for all n samples
-  double *dr = nullptr;
-  float *buf = nullptr;
-  QD_CU(cudaMalloc(&dr, sizeof(double) * 3 * n));
-  const size_t act = (size_t)B * W;
-  const size_t nbuf = (size_t)n * NF + n + (size_t)B * NF + 2 * NL * act + 2 * act + B + 1;
-  cudaError_t e = cudaMalloc(&buf, sizeof(float) * nbuf);
-  if (e != cudaSuccess) { cudaFree(dr); return qd_errf(QD_ERR_NOMEM, "qd_mlp_train: cudaMalloc"); }
-  float *F = buf, *T = F + (size_t)n * NF, *FB = T + n;
-  float *Z = FB + (size_t)B * NF, *A = Z + NL * act;          // [NL][B][64] each
-  float *D = A + NL * act, *D2 = D + act, *Y = D2 + act, *loss = Y + B;
-  std::vector<float> tgt(n);
-  for (int64_t i = 0; i < n; i++) tgt[i] = (float)((V[i] - m->norm.vmean) / m->norm.vstd);
-  int rc = QD_OK;
-  auto fail = [&](cudaError_t x) {
-    rc = qd_errf(QD_ERR_CUDA, "qd_mlp_train: %s", cudaGetErrorString(x));
-  };
-  if ((e = cudaMemcpy(dr, r12, sizeof(double) * n, cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(dr + n, r23, sizeof(double) * n, cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(dr + 2 * n, r13, sizeof(double) * n, cudaMemcpyHostToDevice)) != cudaSuccess ||
-      (e = cudaMemcpy(T, tgt.data(), sizeof(float) * n, cudaMemcpyHostToDevice)) != cudaSuccess)
-    fail(e);
-  if (rc == QD_OK) {
-    k_features<<<(int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096), 256>>>(
-        (int)n, dr, dr + n, dr + 2 * n, m->norm, F);
-    qd_count_launches(1);
-  }
-  // one forward + backward over samples [s0, s0 + b): gradient into d_g
-  auto pass = [&](int64_t s0, int b, float inv_total, bool grads) -> cudaError_t {
-    const float *Fb = F + s0 * NF;
-    const float *tb = T + s0;
-    const int g64 = (b + 63) / 64, gch = (b + GCHUNK - 1) / GCHUNK;
-    for (int l = 0; l < NL; l++) {
-      const int K = l == 0 ? NF : W;
-      const float *in = l == 0 ? Fb : A + (l - 1) * act;
-      k_dense_fwd<<<g64, 256>>>(b, K, in, m->d_wq + layer_off(l), m->d_wq + layer_off(l) + W * K,
-                                Z + l * act, A + l * act);
-    }
-    k_out_loss<<<(b + 7) / 8, 256>>>(b, inv_total, A + (NL - 1) * act, Z + (NL - 1) * act,
-                                     m->d_wq + OFF_WO, m->d_wq + OFF_BO, tb, Y,
-                                     grads ? D : nullptr, loss);
-    qd_count_launches(NL + 1);
-    if (!grads) return cudaGetLastError();
-    k_out_grad<<<gch, 256>>>(b, inv_total, A + (NL - 1) * act, Y, tb, m->d_g + OFF_WO,
-                             m->d_g + OFF_BO);
-    float *Dc = D, *Dn = D2;
-    for (int l = NL - 1; l >= 0; l--) {
-      const int K = l == 0 ? NF : W;
-      const float *in = l == 0 ? Fb : A + (l - 1) * act;
-      k_dense_bwd_weight<<<gch, 256>>>(b, K, Dc, in, m->d_g + layer_off(l),
-                                       m->d_g + layer_off(l) + W * K);
-      if (l > 0) {
-        k_dense_bwd_data<<<g64, 256>>>(b, Dc, m->d_wq + layer_off(l), Z + (l - 1) * act, Dn);
-        float *t = Dc; Dc = Dn; Dn = t;
-      }
-    }
-    qd_count_launches(1 + NL + (NL - 1));
-    return cudaGetLastError();
-  };
-  if (rc == QD_OK && train_steps <= 0) {                      // gradient / loss only
-    cudaMemset(m->d_g, 0, sizeof(float) * NPARAM);
-    cudaMemset(loss, 0, sizeof(float));
-    if ((e = pass(0, (int)n, 1.f / (float)n, grad_out != nullptr)) != cudaSuccess) fail(e);
-    float l = 0.f;
-    if (rc == QD_OK && (e = cudaMemcpy(&l, loss, sizeof(float), cudaMemcpyDeviceToHost)) != cudaSuccess)
-      fail(e);
-    if (rc == QD_OK && grad_out &&
-        (e = cudaMemcpy(grad_out, m->d_g, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost)) != cudaSuccess)
-      fail(e);
-    if (loss_out) *loss_out = l / (double)n;
-  } else if (rc == QD_OK) {
+  // one CTA per tile of the batch, 148 at most (one per SM: 140 KB of shared memory)
+  const int maxrows = (B + TS - 1) / TS < 148 ? (B + TS - 1) / TS : 148;
+  const size_t nd = 4 * (size_t)n;
+  const size_t nf = (size_t)n * NF + n + (size_t)maxrows * PSTRIDE + PSTRIDE + 4;
+  qd_scratch buf(sizeof(double) * nd + sizeof(float) * nf);
+  double *dr = buf.at<double>();
+  if (!dr) return qd_errf(QD_ERR_NOMEM, "qd_mlp_train: %zu bytes", buf.bytes);
+  float *part = reinterpret_cast<float *>(dr + nd);           // 16-byte rows: first after the doubles
+  float *grad = part + (size_t)maxrows * PSTRIDE, *loss = grad + PSTRIDE;
+  float *F = loss + 4, *T = F + (size_t)n * NF;
+  const double *src[4] = {r12, r23, r13, V};
+  for (int q = 0; q < 4; q++)
+    QD_CU(cudaMemcpy(dr + q * n, src[q], sizeof(double) * n, cudaMemcpyHostToDevice));
+  const int gb = (int)((n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096);
+  k_features<<<gb, 256>>>((int)n, dr, dr + n, dr + 2 * n, m->norm, F);
+  k_targets<<<gb, 256>>>(n, dr + 3 * n, m->norm, T);
+  qd_count_launches(2);
+  QD_CU(cudaGetLastError());
+  int64_t counted = n;                                        // samples in *loss
+  if (train_steps <= 0) {                                     // gradient / loss only
+    const float inv = 1.f / (float)n;
+    QD_CU(grad_out ? launch_step<true>(maxrows, (int)n, inv, F, T, m->d_w, part)
+                   : launch_step<false>(maxrows, (int)n, inv, F, T, m->d_w, part));
+    QD_CU(launch_adam(maxrows, part, nullptr, nullptr, nullptr, AdamArgs{}, 1, loss, grad));
+    if (grad_out)
+      QD_CU(cudaMemcpy(grad_out, grad, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
+  } else {
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const double decay = train_steps > 1 ? std::pow(lr_end / lr, 1.0 / (train_steps - 1)) : 1.0;
-    double lr_t = lr, epoch_loss = 0.0;
-    int64_t s0 = 0, seen = 0;
-    cudaMemset(loss, 0, sizeof(float));
-    for (int st = 0; st < train_steps && rc == QD_OK; st++) {
+    double lr_t = lr;
+    int64_t s0 = 0;
+    for (int st = 0; st < train_steps; st++) {
       const int b = (int)(s0 + B <= n ? B : n - s0);
-      cudaMemset(m->d_g, 0, sizeof(float) * NPARAM);
-      if ((e = pass(s0, b, 1.f / (float)b, true)) != cudaSuccess) { fail(e); break; }
+      const int rows = (b + TS - 1) / TS < maxrows ? (b + TS - 1) / TS : maxrows;
+      QD_CU(launch_step<true>(rows, b, 1.f / (float)b, F + s0 * NF, T + s0, m->d_w, part));
       m->step++;
-      const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-      k_adam<<<(NPARAM + 255) / 256, 256>>>(NPARAM, m->d_w, m->d_wq, m->d_g, m->d_m, m->d_v,
-                                            (float)lr_t, b1, b2, eps, c1, c2);
-      qd_count_launches(1);
+      const AdamArgs a{(float)lr_t, b1, b2, eps, 1.f - std::pow(b1, (float)m->step),
+                       1.f - std::pow(b2, (float)m->step)};
+      // the first step of an epoch starts its loss
+      QD_CU(launch_adam(rows, part, m->d_w, m->d_m, m->d_v, a, s0 == 0, loss, nullptr));
       lr_t *= decay;
       s0 += b;
-      seen += b;
-      if (s0 >= n) {                                          // end of an epoch
-        float l = 0.f;
-        cudaMemcpy(&l, loss, sizeof(float), cudaMemcpyDeviceToHost);
-        epoch_loss = l / (double)seen;
-        cudaMemset(loss, 0, sizeof(float));
-        s0 = 0;
-        seen = 0;
-      }
+      counted = s0;
+      if (s0 >= n) s0 = 0;
     }
-    if (rc == QD_OK && (e = cudaDeviceSynchronize()) != cudaSuccess) fail(e);
-    if (seen > 0 && rc == QD_OK) {
-      float l = 0.f;
-      cudaMemcpy(&l, loss, sizeof(float), cudaMemcpyDeviceToHost);
-      epoch_loss = l / (double)seen;
-    }
-    if (loss_out) *loss_out = epoch_loss;
-    if (rc == QD_OK)
-      cudaMemcpy(m->w.data(), m->d_w, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost);
+    m->w.resize(NPARAM);
+    QD_CU(cudaMemcpy(m->w.data(), m->d_w, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost));
   }
-  cudaFree(dr);
-  cudaFree(buf);
-  return rc;
+  float l = 0.f;
+  QD_CU(cudaMemcpy(&l, loss, sizeof(float), cudaMemcpyDeviceToHost));
+  if (loss_out) *loss_out = l / (double)counted;
+  return QD_OK;
 }
 
 // V (hartree) at n geometries (r12, r23, r13 in bohr)
@@ -655,7 +710,7 @@ int qd_mlp_eval(qd_mlp *m, int64_t n, const double *r12, const double *r23, cons
   if (e == cudaSuccess) {
     GridArgs g{};
     const long blocks = (n + 63) / 64;
-    e = launch_mlp_grid(blocks, g, m->norm, m->d_wq, d + 3 * n, n, d, d + n, d + 2 * n);
+    e = launch_mlp_grid(blocks, g, m->norm, m->d_w, d + 3 * n, n, d, d + n, d + 2 * n);
   }
   if (e == cudaSuccess) e = cudaMemcpy(V_out, d + 3 * n, sizeof(double) * n, cudaMemcpyDeviceToHost);
   cudaFree(d);
@@ -686,7 +741,7 @@ int qd_mlp_potential(qd_mlp *m, const qd_radial *R, const qd_radial *r, const qd
   if (e == cudaSuccess) {
     g.R = dR; g.r = dr; g.x = dx;
     const long blocks = (n + 63) / 64;
-    e = launch_mlp_grid(blocks, g, m->norm, m->d_wq, d, n, nullptr, nullptr, nullptr);
+    e = launch_mlp_grid(blocks, g, m->norm, m->d_w, d, n, nullptr, nullptr, nullptr);
   }
   if (e == cudaSuccess) e = cudaMemcpy(pot_out, d, sizeof(double) * n, cudaMemcpyDeviceToHost);
   cudaFree(d);

@@ -30,6 +30,7 @@
 #include <emmintrin.h>
 #endif
 #include "qd.h"
+#include "qd_err.h"
 #include "qd_kernels.h"
 #include "qd_tc.h"
 
@@ -534,6 +535,36 @@ int qd_set_error(int code, const char *msg)
   return code;
 }
 void qd_count_launches(int n) { g_launches += n; }
+
+// call scratch (qd_err.h): one pool per device, made on first use
+cudaError_t qd_scratch_alloc(void **p, size_t bytes)
+{
+  constexpr int MAXDEV = 64;
+  static std::mutex mu;
+  static cudaMemPool_t pools[MAXDEV] = {};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev >= MAXDEV) return cudaErrorInvalidDevice;
+  cudaMemPool_t pool;
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    if (!pools[dev]) {
+      cudaMemPoolProps props = {};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      cudaMemPool_t made;
+      e = cudaMemPoolCreate(&made, &props);
+      if (e != cudaSuccess) return e;
+      uint64_t keep = QD_SCRATCH_KEEP;
+      cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep);
+      pools[dev] = made;
+    }
+    pool = pools[dev];
+  }
+  return cudaMallocFromPoolAsync(p, bytes, pool, 0);
+}
 
 struct qd_handle {
   int dev = 0;                    // the device current at creation: its stream and buffers

@@ -1,4 +1,5 @@
-// qd_err.h -- error reporting shared by the library's translation units.
+// qd_err.h -- error reporting and call scratch shared by the library's
+// translation units.
 #pragma once
 #include <cstdarg>
 #include <cstdio>
@@ -25,3 +26,29 @@ inline int qd_errf(int code, const char *fmt, ...)
       return qd_errf(QD_ERR_CUDA, "%s failed: %s (%s:%d)", #x, cudaGetErrorString(e_),   \
                      __FILE__, __LINE__);                                               \
   } while (0)
+
+// Device memory of one call (the set-up entry points, which work on the legacy
+// default stream): allocated on construction, returned to the pool on
+// destruction, in stream order.  The pool keeps at most QD_SCRATCH_KEEP bytes
+// between calls and belongs to the current device, so a call does not pay
+// cudaMalloc and cudaFree (0.2-0.5 ms together, and a device-wide wait).
+constexpr size_t QD_SCRATCH_KEEP = size_t(256) << 20;
+cudaError_t qd_scratch_alloc(void **p, size_t bytes);
+struct qd_scratch {
+  void *p = nullptr;
+  size_t bytes;
+  explicit qd_scratch(size_t n) : bytes(n)
+  {
+    if (qd_scratch_alloc(&p, n) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+    }
+  }
+  ~qd_scratch()
+  {
+    if (p) cudaFreeAsync(p, 0);
+  }
+  qd_scratch(const qd_scratch &) = delete;
+  qd_scratch &operator=(const qd_scratch &) = delete;
+  template <typename T> T *at() const { return static_cast<T *>(p); }
+};
