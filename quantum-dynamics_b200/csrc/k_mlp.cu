@@ -20,7 +20,7 @@
 // k_mlp_adam sums the rows in order and updates the weights.  (One launch per
 // layer and direction, activations in global memory and the weight gradients
 // on 8 CTAs with atomics, took 342 us a step at 4096 samples; this form takes 22.)
-// Inference: one fused kernel per tile of 64 points (features from the
+// Inference: one fused kernel per tile of 256 points (features from the
 // Jacobi geometry, all layers in shared memory).
 #include <cmath>
 #include <cstring>
@@ -391,36 +391,70 @@ cudaError_t launch_adam(int rows, const float *part, float *w, float *m, float *
 }
 
 // Fused inference on the Jacobi grid (H3/H3PESJacobi.m:5-27 geometry): per
-// tile of 64 points, features, four SiLU layers and the output in shared
-// memory; V = vmax where a distance <= rmin, else min(V_mlp, vmax) if cap.
+// tile of points, features, four SiLU layers and the output in shared memory;
+// V = vmax where a distance <= rmin, else min(V_mlp, vmax) if cap.
 struct GridArgs {
   int n1, n2, nth;
   const double *R, *r, *x;
   double f2, f3, vmax, rmin;
   int cap;
 };
-// every layer's weights stay in shared memory for the whole launch (loaded
-// once per CTA), activations of 64 points at a time in place
-constexpr int WS = W + 1;                                  // padded weight / activation row
-constexpr size_t GRID_SMEM = sizeof(float) * ((size_t)NL * W * WS + 64 * WS + 64 * NF) + 64;
-__global__ void __launch_bounds__(256) k_mlp_grid(GridArgs g, Norm nm, const float *wq,
-                                                  double *pot, long npts, const double *r12p,
-                                                  const double *r23p, const double *r13p)
+// Every layer's weights stay in shared memory for the whole launch (loaded once
+// per CTA), activations of GP points at a time in place, transposed ([k][point]).
+// A thread forms 8 points x 4 outputs as paired FP32 FMAs (fma.rn.f32x2, two
+// points a register pair): per k, 2 16-byte loads of activations and 2 of
+// weights, which are stored twice each so that a pair (w, w) is one load, for 16
+// paired FMAs.  Bound: the products and the SiLUs together (12.4 kFMA per point,
+// 0.36 ms at the FP32 rate on 128 x 128 x 64, and 256 exponentials and divisions
+// a point, as many instructions as the paired FMAs).  There: scalar FMAs, 4 x 4
+// outputs a thread with scalar loads 1.18 ms; 8 x 4 with 16-byte loads 0.96 ms;
+// this form 0.91 ms.
+constexpr int GP = 256, GT = 512;
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b)
+{
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v)
+{
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+struct GridSmem {
+  float2 w[NL - 1][W][W];                 // layers 2..4: [k][o], each weight twice
+  float h[W][GP];                         // activations
+  float w1[W][NF], b[NL][W], wo[W];
+  float f[GP][NF];
+  unsigned char mask[GP];
+};
+__global__ void __launch_bounds__(GT, 1) k_mlp_grid(GridArgs g, Norm nm, const float *wq,
+                                                    double *pot, long npts, const double *r12p,
+                                                    const double *r23p, const double *r13p)
 {
   extern __shared__ float4 grid_sm4[];
-  float *sm = reinterpret_cast<float *>(grid_sm4);
-  float (*Wsm)[W][WS] = reinterpret_cast<float (*)[W][WS]>(sm);            // [NL][W][WS]
-  float (*H)[WS] = reinterpret_cast<float (*)[WS]>(sm + NL * W * WS);      // [64][WS]
-  float (*feat)[NF] = reinterpret_cast<float (*)[NF]>(sm + NL * W * WS + 64 * WS);
-  unsigned char *mask = reinterpret_cast<unsigned char *>(sm + NL * W * WS + 64 * WS + 64 * NF);
-  const int tid = threadIdx.x, tr = tid >> 4, tc = tid & 15;
-  for (int l = 0; l < NL; l++) {
-    const int K = l == 0 ? NF : W;
-    const float *Wl = wq + layer_off(l);
-    for (int x = tid; x < W * K; x += 256) Wsm[l][x / K][x % K] = Wl[x];
+  GridSmem &m = *reinterpret_cast<GridSmem *>(grid_sm4);
+  const int tid = threadIdx.x, tp = tid & 31, to = tid >> 5;   // points 4 tp.., 128 + 4 tp..; outputs 4 to..
+  for (int x = tid; x < (NL - 1) * W * W; x += GT) {
+    const int l = x / (W * W), k = x / W % W, o = x % W;
+    const float v = wq[layer_off(l + 1) + o * W + k];
+    m.w[l][k][o] = make_float2(v, v);
   }
-  for (long base = (long)blockIdx.x * 64; base < npts; base += (long)gridDim.x * 64) {
-    if (tid < 64) {
+  for (int x = tid; x < W * NF; x += GT) m.w1[x / NF][x % NF] = wq[x];
+  for (int x = tid; x < NL * W; x += GT)
+    m.b[x / W][x % W] = wq[layer_off(x / W) + W * (x / W ? W : NF) + x % W];
+  if (tid < W) m.wo[tid] = wq[OFF_WO + tid];
+  const float bo = wq[OFF_BO];
+  for (long base = (long)blockIdx.x * GP; base < npts; base += (long)gridDim.x * GP) {
+    if (tid < GP) {
       const long q = base + tid;
       float f[NF] = {0.f, 0.f, 0.f};
       unsigned char ok = 0;
@@ -440,46 +474,64 @@ __global__ void __launch_bounds__(256) k_mlp_grid(GridArgs g, Norm nm, const flo
         }
         features((float)r12, (float)r23, (float)r13, nm, f);
       }
-      for (int c = 0; c < NF; c++) feat[tid][c] = f[c];
-      mask[tid] = ok;
+      for (int c = 0; c < NF; c++) m.f[tid][c] = f[c];
+      m.mask[tid] = ok;
     }
     __syncthreads();                      // features (and, first time, the weights) in place
-    for (int l = 0; l < NL; l++) {
-      const int K = l == 0 ? NF : W;
-      const float *bl = wq + layer_off(l) + W * K;
-      float acc[4][4];
+    {
+      const int s = tid % GP;
+      const float f0 = m.f[s][0], f1 = m.f[s][1], f2 = m.f[s][2];
+#pragma unroll 4
+      for (int o = tid / GP; o < W; o += GT / GP)
+        m.h[o][s] = silu(fmaf(f2, m.w1[o][2], fmaf(f1, m.w1[o][1], fmaf(f0, m.w1[o][0], m.b[0][o]))));
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int l = 1; l < NL; l++) {
+      f32x2 acc[4][4];                    // point pairs x outputs
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int j = 0; j < 4; j++) {
+        const float bj = m.b[l][4 * to + j];
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = bl[tc + 16 * j];
-      for (int k = 0; k < K; k++) {
-        float a[4], w[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) a[i] = l == 0 ? feat[tr + 16 * i][k] : H[tr + 16 * i][k];
-#pragma unroll
-        for (int j = 0; j < 4; j++) w[j] = Wsm[l][tc + 16 * j][k];
+        for (int i = 0; i < 4; i++) acc[i][j] = pack2(bj, bj);
+      }
+#pragma unroll 4
+      for (int k = 0; k < W; k++) {
+        const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(&m.h[k][4 * tp]);
+        const ulonglong2 a1 = *reinterpret_cast<const ulonglong2 *>(&m.h[k][GP / 2 + 4 * tp]);
+        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2 *>(&m.w[l - 1][k][4 * to]);
+        const ulonglong2 w1 = *reinterpret_cast<const ulonglong2 *>(&m.w[l - 1][k][4 * to + 2]);
+        const f32x2 a[4] = {a0.x, a0.y, a1.x, a1.y}, w[4] = {w0.x, w0.y, w1.x, w1.y};
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] = fmaf(a[i], w[j], acc[i][j]);
+          for (int j = 0; j < 4; j++) acc[i][j] = fma2(a[i], w[j], acc[i][j]);
       }
-      __syncthreads();                    // every read of H is done
+      __syncthreads();                    // every read of the activations is done
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int j = 0; j < 4; j++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) H[tr + 16 * i][tc + 16 * j] = silu(acc[i][j]);
+        for (int i = 0; i < 4; i += 2) {
+          const float2 u = unpack2(acc[i][j]), v = unpack2(acc[i + 1][j]);
+          *reinterpret_cast<float4 *>(&m.h[4 * to + j][(i ? GP / 2 : 0) + 4 * tp]) =
+              make_float4(silu(u.x), silu(u.y), silu(v.x), silu(v.y));
+        }
       __syncthreads();
     }
-    // output: one warp per 8 points
-    const int lane = tid & 31, warp = tid >> 5;
-    for (int pnt = warp; pnt < 64; pnt += 8) {
-      float acc = H[pnt][lane] * wq[OFF_WO + lane] + H[pnt][lane + 32] * wq[OFF_WO + lane + 32];
-      for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      const long q = base + pnt;
-      if (lane == 0 && q < npts) {
-        double v = (double)(acc + wq[OFF_BO]) * nm.vstd + nm.vmean;
+    if (tid < GP) {                       // output: one thread a point, halves folded pairwise
+      float p[W / 2];
+#pragma unroll
+      for (int k = 0; k < W / 2; k++)
+        p[k] = m.h[k][tid] * m.wo[k] + m.h[k + W / 2][tid] * m.wo[k + W / 2];
+#pragma unroll
+      for (int o = W / 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < o; k++) p[k] += p[k + o];
+      const long q = base + tid;
+      if (q < npts) {
+        double v = (double)(p[0] + bo) * nm.vstd + nm.vmean;
         if (!r12p) {
-          if (!mask[pnt]) v = g.vmax;
+          if (!m.mask[tid]) v = g.vmax;
           else if (g.cap) v = fmin(v, g.vmax);
         }
         pot[q] = v;
@@ -489,14 +541,14 @@ __global__ void __launch_bounds__(256) k_mlp_grid(GridArgs g, Norm nm, const flo
   }
 }
 
-cudaError_t launch_mlp_grid(long blocks, const GridArgs &g, const Norm &nm, const float *wq,
-                            double *pot, long npts, const double *r12p, const double *r23p,
-                            const double *r13p)
+cudaError_t launch_mlp_grid(const GridArgs &g, const Norm &nm, const float *wq, double *pot,
+                            long npts, const double *r12p, const double *r23p, const double *r13p)
 {
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_mlp_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GRID_SMEM);
-  if (attr != cudaSuccess) return attr;
-  k_mlp_grid<<<(unsigned)(blocks < 148 * 2 ? blocks : 148 * 2), 256, GRID_SMEM>>>(
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_mlp_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GridSmem));
+  if (e != cudaSuccess) return e;
+  const long blocks = (npts + GP - 1) / GP;
+  k_mlp_grid<<<(unsigned)(blocks < 148 ? blocks : 148), GT, sizeof(GridSmem)>>>(
       g, nm, wq, pot, npts, r12p, r23p, r13p);
   qd_count_launches(1);
   return cudaGetLastError();
@@ -702,18 +754,17 @@ int qd_mlp_eval(qd_mlp *m, int64_t n, const double *r12, const double *r23, cons
                 double *V_out)
 {
   if (!m || n < 1 || !r12 || !r23 || !r13 || !V_out) return qd_errf(QD_ERR_INVALID, "bad argument");
-  double *d = nullptr;
-  QD_CU(cudaMalloc(&d, sizeof(double) * 4 * n));
+  qd_scratch buf(sizeof(double) * 4 * (size_t)n);
+  double *d = buf.at<double>();
+  if (!d) return qd_errf(QD_ERR_NOMEM, "qd_mlp_eval: %zu bytes of device memory", buf.bytes);
   cudaError_t e = cudaMemcpy(d, r12, sizeof(double) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d + n, r23, sizeof(double) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d + 2 * n, r13, sizeof(double) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
     GridArgs g{};
-    const long blocks = (n + 63) / 64;
-    e = launch_mlp_grid(blocks, g, m->norm, m->d_w, d + 3 * n, n, d, d + n, d + 2 * n);
+    e = launch_mlp_grid(g, m->norm, m->d_w, d + 3 * n, n, d, d + n, d + 2 * n);
   }
-  if (e == cudaSuccess) e = cudaMemcpy(V_out, d + 3 * n, sizeof(double) * n, cudaMemcpyDeviceToHost);
-  cudaFree(d);
+  if (e == cudaSuccess) e = qd_fetch(V_out, d + 3 * n, sizeof(double) * n);
   if (e != cudaSuccess) return qd_errf(QD_ERR_CUDA, "qd_mlp_eval: %s", cudaGetErrorString(e));
   return QD_OK;
 }
@@ -732,19 +783,18 @@ int qd_mlp_potential(qd_mlp *m, const qd_radial *R, const qd_radial *r, const qd
   g.f3 = 1.0 - g.f2;
   g.vmax = vmax; g.rmin = rmin; g.cap = cap ? 1 : 0;
   const long n = (long)g.n1 * g.n2 * g.nth;
-  double *d = nullptr;
-  QD_CU(cudaMalloc(&d, sizeof(double) * ((size_t)n + g.n1 + g.n2 + g.nth)));
+  qd_scratch buf(sizeof(double) * ((size_t)n + g.n1 + g.n2 + g.nth));
+  double *d = buf.at<double>();
+  if (!d) return qd_errf(QD_ERR_NOMEM, "qd_mlp_potential: %zu bytes of device memory", buf.bytes);
   double *dR = d + n, *dr = dR + g.n1, *dx = dr + g.n2;
   cudaError_t e = cudaMemcpy(dR, R->r, sizeof(double) * g.n1, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(dr, r->r, sizeof(double) * g.n2, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(dx, theta->x, sizeof(double) * g.nth, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) {
     g.R = dR; g.r = dr; g.x = dx;
-    const long blocks = (n + 63) / 64;
-    e = launch_mlp_grid(blocks, g, m->norm, m->d_w, d, n, nullptr, nullptr, nullptr);
+    e = launch_mlp_grid(g, m->norm, m->d_w, d, n, nullptr, nullptr, nullptr);
   }
-  if (e == cudaSuccess) e = cudaMemcpy(pot_out, d, sizeof(double) * n, cudaMemcpyDeviceToHost);
-  cudaFree(d);
+  if (e == cudaSuccess) e = qd_fetch(pot_out, d, sizeof(double) * n);
   if (e != cudaSuccess) return qd_errf(QD_ERR_CUDA, "qd_mlp_potential: %s", cudaGetErrorString(e));
   return QD_OK;
 }

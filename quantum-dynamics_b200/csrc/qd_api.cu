@@ -335,7 +335,7 @@ class Staging {
     size_t bytes;         // device bytes
     bool widen = false;   // src holds floats, dst receives them as doubles (2 x bytes)
   };
-  cudaError_t download(const Piece *pc, int np, cudaStream_t st)
+  cudaError_t download(const Piece *pc, int np, cudaStream_t st, size_t least = LARGE)
   {
     std::lock_guard<std::mutex> lock(mu_);
     size_t total = 0;
@@ -345,7 +345,7 @@ class Staging {
       widen = widen || pc[i].widen;
     }
     if (widen && !ready()) return cudaErrorMemoryAllocation;
-    if (!widen && (!ready() || (np == 1 && total < LARGE))) {
+    if (!widen && (!ready() || (np == 1 && total < least))) {
       for (int i = 0; i < np; i++) {
         cudaError_t e = cudaMemcpyAsync(pc[i].dst, pc[i].src, pc[i].bytes, cudaMemcpyDeviceToHost,
                                         st);
@@ -535,6 +535,12 @@ int qd_set_error(int code, const char *msg)
   return code;
 }
 void qd_count_launches(int n) { g_launches += n; }
+
+cudaError_t qd_fetch(void *dst, const void *src, size_t bytes)
+{
+  const Staging::Piece one{dst, src, bytes};
+  return Staging::get().download(&one, 1, 0, size_t(256) << 10);
+}
 
 // call scratch (qd_err.h): one pool per device, made on first use
 cudaError_t qd_scratch_alloc(void **p, size_t bytes)

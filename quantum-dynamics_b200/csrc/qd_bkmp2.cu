@@ -269,8 +269,9 @@ int qd_bkmp2_eval(int64_t n, const double *r1, const double *r2, const double *r
 {
   if (n > 0 && (!r1 || !r2 || !r3 || !v_out)) return qd_errf(QD_ERR_INVALID, "NULL argument");
   if (n <= 0) return QD_OK;
-  double *d = nullptr;
-  QD_CU(cudaMalloc(&d, sizeof(double) * 4 * (size_t)n));
+  qd_scratch buf(sizeof(double) * 4 * (size_t)n);
+  double *d = buf.at<double>();
+  if (!d) return qd_errf(QD_ERR_NOMEM, "qd_bkmp2_eval: %zu bytes of device memory", buf.bytes);
   cudaError_t e = cudaMemcpy(d, r1, sizeof(double) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d + n, r2, sizeof(double) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d + 2 * n, r3, sizeof(double) * n, cudaMemcpyHostToDevice);
@@ -281,8 +282,7 @@ int qd_bkmp2_eval(int64_t n, const double *r1, const double *r2, const double *r
     qd_count_launches(1);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpy(v_out, d + 3 * n, sizeof(double) * n, cudaMemcpyDeviceToHost);
-  cudaFree(d);
+  if (e == cudaSuccess) e = qd_fetch(v_out, d + 3 * n, sizeof(double) * n);
   if (e != cudaSuccess) return qd_errf(QD_ERR_CUDA, "qd_bkmp2_eval: %s", cudaGetErrorString(e));
   return QD_OK;
 }
@@ -304,8 +304,9 @@ int qd_potential_bkmp2(const qd_radial *R, const qd_radial *r, const qd_angle *t
   g.f3 = 1.0 - g.f2;
   g.vmax = vmax; g.rmin = rmin; g.cap = cap ? 1 : 0;
   const long n = (long)g.n1 * g.n2 * g.nth;
-  double *d = nullptr;
-  QD_CU(cudaMalloc(&d, sizeof(double) * ((size_t)n + g.n1 + g.n2 + g.nth)));
+  qd_scratch buf(sizeof(double) * ((size_t)n + g.n1 + g.n2 + g.nth));
+  double *d = buf.at<double>();
+  if (!d) return qd_errf(QD_ERR_NOMEM, "qd_potential_bkmp2: %zu bytes of device memory", buf.bytes);
   double *dR = d + n, *dr = dR + g.n1, *dx = dr + g.n2;
   cudaError_t e = cudaMemcpy(dR, R->r, sizeof(double) * g.n1, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(dr, r->r, sizeof(double) * g.n2, cudaMemcpyHostToDevice);
@@ -317,8 +318,7 @@ int qd_potential_bkmp2(const qd_radial *R, const qd_radial *r, const qd_angle *t
     qd_count_launches(1);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpy(pot_out, d, sizeof(double) * n, cudaMemcpyDeviceToHost);
-  cudaFree(d);
+  if (e == cudaSuccess) e = qd_fetch(pot_out, d, sizeof(double) * n);
   if (e != cudaSuccess) return qd_errf(QD_ERR_CUDA, "qd_potential_bkmp2: %s", cudaGetErrorString(e));
   return QD_OK;
 }

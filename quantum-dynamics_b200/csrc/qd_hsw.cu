@@ -469,8 +469,9 @@ int qd_hsw_eval(const qd_hsw *h, int64_t n, const double *r_fh1, const double *r
   if (!h || (n > 0 && (!r_fh1 || !r_hh || !r_fh2 || !v_out)))
     return qd_errf(QD_ERR_INVALID, "NULL argument");
   if (n <= 0) return QD_OK;
-  double *d = nullptr;
-  QD_CU(cudaMalloc(&d, sizeof(double) * 4 * (size_t)n));
+  qd_scratch buf(sizeof(double) * 4 * (size_t)n);
+  double *d = buf.at<double>();
+  if (!d) return qd_errf(QD_ERR_NOMEM, "qd_hsw_eval: %zu bytes of device memory", buf.bytes);
   cudaError_t e = cudaMemcpy(d, r_fh1, sizeof(double) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d + n, r_hh, sizeof(double) * n, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(d + 2 * n, r_fh2, sizeof(double) * n, cudaMemcpyHostToDevice);
@@ -481,8 +482,7 @@ int qd_hsw_eval(const qd_hsw *h, int64_t n, const double *r_fh1, const double *r
     qd_count_launches(1);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpy(v_out, d + 3 * n, sizeof(double) * n, cudaMemcpyDeviceToHost);
-  cudaFree(d);
+  if (e == cudaSuccess) e = qd_fetch(v_out, d + 3 * n, sizeof(double) * n);
   if (e != cudaSuccess) return qd_errf(QD_ERR_CUDA, "qd_hsw_eval: %s", cudaGetErrorString(e));
   return QD_OK;
 }
@@ -503,8 +503,9 @@ int qd_potential_hsw(const qd_radial *R, const qd_radial *r, const qd_angle *the
   g.f3 = 1.0 - g.f2;
   g.vmax = vmax; g.rmin = rmin; g.cap = cap ? 1 : 0;
   const long n = (long)g.n1 * g.n2 * g.nth;
-  double *d = nullptr;
-  QD_CU(cudaMalloc(&d, sizeof(double) * ((size_t)n + g.n1 + g.n2 + g.nth)));
+  qd_scratch buf(sizeof(double) * ((size_t)n + g.n1 + g.n2 + g.nth));
+  double *d = buf.at<double>();
+  if (!d) return qd_errf(QD_ERR_NOMEM, "qd_potential_hsw: %zu bytes of device memory", buf.bytes);
   double *dR = d + n, *dr = dR + g.n1, *dx = dr + g.n2;
   cudaError_t e = cudaMemcpy(dR, R->r, sizeof(double) * g.n1, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(dr, r->r, sizeof(double) * g.n2, cudaMemcpyHostToDevice);
@@ -516,8 +517,7 @@ int qd_potential_hsw(const qd_radial *R, const qd_radial *r, const qd_angle *the
     qd_count_launches(1);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpy(pot_out, d, sizeof(double) * n, cudaMemcpyDeviceToHost);
-  cudaFree(d);
+  if (e == cudaSuccess) e = qd_fetch(pot_out, d, sizeof(double) * n);
   if (e != cudaSuccess) return qd_errf(QD_ERR_CUDA, "qd_potential_hsw: %s", cudaGetErrorString(e));
   return QD_OK;
 }

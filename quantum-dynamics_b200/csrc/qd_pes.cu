@@ -140,8 +140,9 @@ int qd_potential_leps(const qd_radial *R, const qd_radial *r, const qd_angle *th
     p.pf[s] = 0.5 * pr[s]->de * (1.0 - pr[s]->sato) / (1.0 + pr[s]->sato);
   }
   const long n = (long)g.n1 * g.n2 * g.nth;
-  double *d = nullptr;
-  QD_CU(cudaMalloc(&d, sizeof(double) * ((size_t)n + g.n1 + g.n2 + g.nth)));
+  qd_scratch buf(sizeof(double) * ((size_t)n + g.n1 + g.n2 + g.nth));
+  double *d = buf.at<double>();
+  if (!d) return qd_errf(QD_ERR_NOMEM, "qd_potential_leps: %zu bytes of device memory", buf.bytes);
   double *dR = d + n, *dr = dR + g.n1, *dx = dr + g.n2;
   cudaError_t e = cudaMemcpy(dR, g.R, sizeof(double) * g.n1, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(dr, g.r, sizeof(double) * g.n2, cudaMemcpyHostToDevice);
@@ -154,8 +155,7 @@ int qd_potential_leps(const qd_radial *R, const qd_radial *r, const qd_angle *th
     qd_count_launches(1);
     e = cudaGetLastError();
   }
-  if (e == cudaSuccess) e = cudaMemcpy(pot_out, d, sizeof(double) * n, cudaMemcpyDeviceToHost);
-  cudaFree(d);
+  if (e == cudaSuccess) e = qd_fetch(pot_out, d, sizeof(double) * n);
   if (e != cudaSuccess) return qd_errf(QD_ERR_CUDA, "qd_potential_leps: %s", cudaGetErrorString(e));
   return QD_OK;
 }
