@@ -4,7 +4,7 @@
 //     expV[k][j][i] = exp(-i V dt)                       setup_exp_ipot_dt    timeEvol.C:438-463
 //     rot[l][j][i]  = exp(-i l(l+1)(I1_i + I2_j) dt/2)   setup_exp_irot_dt_2  timeEvol.C:465-491
 //     kin[j][i]     = exp(-i(T1_i + T2_j) dt) / n1 / n2  setup_exp_ikin_dt    timeEvol.C:493-517
-//   or, for the kernels of k_axis.cuh, the factors of rot and kin in R and in r
+//   or, for the kernels of k_axis_f64.cu, the factors of rot and kin in R and in r
 //   FP32 form: exp(-i V dt) and the separable factors of the rotational and
 //   kinetic phases (exp(-i l(l+1) I1 dt/2), exp(-i l(l+1) I2 dt/2),
 //   exp(-i T1 dt), exp(-i T2 dt)), each evaluated in FP64 with the phase

@@ -11,8 +11,8 @@
 // shared memory (plain ld/st to the peers' shared memory, cluster barriers
 // around each exchange).  psi_l is read and written once per step.
 //
-// It serves the grids that neither k_slice_rf.cu nor k_axis.cuh takes (a size
-// that is not a product of two of their radices, such as 18 or 250).
+// It serves the grids that neither k_slice_rf.cu nor k_axis_f32.cu takes (a
+// size that is not two groups of radices, such as 8 or 162).
 //
 // FFTs are shared-memory Stockham passes (radix 8/4/2/3/5 in registers).
 // Row buffers are padded by one element per 8 so that the radix-8 output
@@ -222,10 +222,7 @@ template <int CL> cudaError_t launch_cl(const LineParams &p, cudaStream_t s)
 
 int slice_cluster_ok(int n1, int n2, int cl)
 {
-  if (slice_is_ax(cl)) {
-    AxisPlan ax;
-    return axis_plan(n1, n2, sizeof(float2), cl == SLICE_AX, ax) ? 1 : 0;
-  }
+  if (cl == SLICE_AX) return axis_f32_ok(n1, n2) ? 1 : 0;
   if (cl == SLICE_RF4W) return slice_rf_wide_ok(n1, n2) ? 1 : 0;
   if (slice_is_rf(cl)) return slice_rf_threads(n1, n2, slice_ctas(cl)) > 0;
   if (cl != 1 && cl != 2 && cl != 4) return 0;
@@ -235,7 +232,7 @@ int slice_cluster_ok(int n1, int n2, int cl)
 
 int slice_threads(int n1, int n2, int cl)
 {
-  if (slice_is_ax(cl)) return axis_threads(cl);
+  if (cl == SLICE_AX) return axis_threads();
   return slice_is_rf(cl) ? slice_rf_threads(n1, n2, slice_ctas(cl)) : NT;
 }
 
@@ -246,8 +243,7 @@ cudaError_t launch_slice(const LineParams &p, cudaStream_t s)
     case SLICE_RF2: return launch_slice_rf(p, 2, s);
     case SLICE_RF4: return launch_slice_rf(p, 4, s);
     case SLICE_RF4W: return launch_slice_rf_wide(p, s);
-    case SLICE_AX:
-    case SLICE_AX2: return launch_axis_f32(p, s);
+    case SLICE_AX: return launch_axis_f32(p, s);
     case 1: return launch_cl<1>(p, s);
     case 2: return launch_cl<2>(p, s);
     case 4: return launch_cl<4>(p, s);

@@ -600,6 +600,7 @@ struct qd_handle {
   double2 *d_expV = nullptr, *d_rot = nullptr, *d_kin = nullptr;
   double2 *d_zr1 = nullptr, *d_zr2 = nullptr, *d_zk1 = nullptr, *d_zk2 = nullptr;
   float2 *d_expV32 = nullptr;
+  float2 *d_ts1 = nullptr, *d_ts2 = nullptr;
   float2 *d_rc1 = nullptr, *d_rc2 = nullptr, *d_kc1 = nullptr, *d_kc2 = nullptr;
   int slice_cluster = 0;          // l-space kernel (LineParams::cluster code)
   int flux_variant = 0;           // flux-accumulation GEMM tile variant (tune_flux)
@@ -919,6 +920,7 @@ LineParams line_params(qd_handle *h, bool f32)
   p.nruns = h->nruns;
   p.rot = h->d_rot; p.kin = h->d_kin;
   p.rc1 = h->d_rc1; p.rc2 = h->d_rc2; p.kc1 = h->d_kc1; p.kc2 = h->d_kc2;
+  p.ts1 = h->d_ts1; p.ts2 = h->d_ts2;
   p.zr1 = h->d_zr1; p.zr2 = h->d_zr2; p.zk1 = h->d_zk1; p.zk2 = h->d_zk2;
   p.cluster = h->slice_cluster;
   const double ks = 1.0 / ((double)h->n1 * h->n2);
@@ -939,61 +941,50 @@ cudaError_t run_lines(const LineParams &p, bool f32, cudaStream_t st)
   return p.cluster ? launch_axis_f64(p, st) : launch_lines<double>(p, st);
 }
 
-// the FP64 l-space kernels beside the split ones: k_axis.cuh, where it takes
-// the grid (QD_SLICE_CLUSTER=0 keeps the split kernels)
-bool axis_f64(const qd_handle *h, bool fused)
+// FP64 l-space pass on k_axis_f64.cu, where it takes the grid
+// (QD_SLICE_CLUSTER=0 keeps the split kernels)
+bool axis_f64(const qd_handle *h)
 {
-  AxisPlan ax;
   const char *force = getenv("QD_SLICE_CLUSTER");
-  return !(force && atoi(force) == 0) &&
-         axis_plan(h->n1, h->n2, sizeof(double2), fused, ax);
+  return !(force && atoi(force) == 0) && axis_f64_ok(h->n1, h->n2);
 }
 
-// Autotuner of the l-space pass: time the kernels that take the grid on the
-// handle's zero l-space buffer (a zero wavepacket stays zero) and keep the
-// fastest; the choice is kept for later handles of the same shapes.  The kernels that are tried, per grid:
+// Choice of the l-space kernel.
 //   complex64, sizes compiled in: the register-FFT slice kernel on 1, 2 or 4
-//     CTAs per slice (128 x 96 x 64, one run: 14.8 us a step on two; run-time
-//     sizes 19.0, Stockham slice kernel 22.8);
-//   two built factors a side (k_axis.cuh): its fused form and its row and
-//     column launches, either of which may win (54 x 60 x 32 complex64: 15.8
-//     and 17.1 us; 144 x 120 x 64: 35 and 23 us; the Stockham kernels 25 and 51);
-//   other grids: the split kernels and (complex64) the Stockham slice kernel
-//     on 1, 2 and 4 CTAs per slice.
-// QD_SLICE_CLUSTER=0|1|2|4|8|9|10|11|12|13 forces a choice (0 the split
-// kernels, 1, 2, 4 the Stockham slice kernel, 8, 9, 10 the register-FFT kernel
-// on 1, 2 and 4 CTAs, 11 its wide form, 12, 13 the run-time one, fused or as two
-// launches; FP64 knows 0, 12 and 13 only).
+//     CTAs per slice, timed on the handle's zero l-space buffer (a zero
+//     wavepacket stays zero), the choice kept for later handles of the shapes;
+//   sizes that k_axis_f32.cu / k_axis_f64.cu take: those (complex64, us a step,
+//     the best Stockham form -> k_axis_f32: 48 x 40 x 24 16.3 -> 16.5, 54 x 60 x 32
+//     25 -> 17.5, 144 x 120 x 64 52 -> 25, 200 x 180 x 40 93 -> 36, 8 runs of
+//     96 x 96 x 48 105 -> 54; FP64: k_axis_f64.cu);
+//   other grids: FP64 the split kernels; complex64 the split kernels or the
+//     Stockham slice kernel on 1, 2 or 4 CTAs per slice, timed likewise.
+// QD_SLICE_CLUSTER=0|1|2|4|8|9|10|11|12 forces a choice (0 the split kernels,
+// 1, 2, 4 the Stockham slice kernel, 8, 9, 10 the register-FFT kernel on 1, 2
+// and 4 CTAs, 11 its wide form, 12 the run-time register-FFT kernels; FP64 knows
+// 0 and 12 only).
 int tune_slice(qd_handle *h)
 {
-  h->slice_cluster = 0;
   const bool f32 = h->prec == QD_PREC_FP32;
-  auto built = [&](int cl) {
-    return f32 ? slice_cluster_ok(h->n1, h->n2, cl) != 0
-               : slice_is_ax(cl) && axis_f64(h, cl == SLICE_AX);
-  };
-  const bool rf = f32 && (built(SLICE_RF) || built(SLICE_RF2) || built(SLICE_RF4));
-  const bool ax = !rf && built(SLICE_AX2);
-  auto tried = [&](int cl) {
-    return rf ? slice_is_rf(cl) && built(cl) : ax ? slice_is_ax(cl) && built(cl)
-                                                 : cl == 0 || (!slice_is_ax(cl) && built(cl));
-  };
-  const char *force = getenv("QD_SLICE_CLUSTER");
-  const int forced = force ? atoi(force) : 0;
-  if (force && (f32 || forced == 0 || slice_is_ax(forced))) {
-    if (forced) h->slice_cluster = built(forced) ? forced : 0;
-    if (f32 || forced == 0 || h->slice_cluster) return QD_OK;
+  h->slice_cluster = !f32 && axis_f64(h) ? SLICE_AX : 0;
+  if (!f32) return QD_OK;
+  auto built = [&](int cl) { return slice_cluster_ok(h->n1, h->n2, cl) != 0; };
+  if (const char *force = getenv("QD_SLICE_CLUSTER")) {
+    const int cl = atoi(force);
+    h->slice_cluster = built(cl) ? cl : 0;
+    return QD_OK;
   }
-  if (!f32) {
-    if (!ax) return QD_OK;
-    h->slice_cluster = SLICE_AX2;       // the tables of the split kernels are not built
+  const bool rf = built(SLICE_RF) || built(SLICE_RF2) || built(SLICE_RF4);
+  if (!rf && built(SLICE_AX)) {
+    h->slice_cluster = SLICE_AX;
+    return QD_OK;
   }
   // the choice depends on the shapes only: measured once per process and device
   static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int, int, int, int, int>, int> chosen;
+  static std::map<std::tuple<int, int, int, int, int, int, int>, int> chosen;
   int dev = 0;
   cudaGetDevice(&dev);
-  const auto key = std::make_tuple(dev, h->prec, h->n1, h->n2, h->nl, h->nruns, h->jrows,
+  const auto key = std::make_tuple(dev, h->n1, h->n2, h->nl, h->nruns, h->jrows,
                                    h->d_run_k ? 1 : 0);
   {
     std::lock_guard<std::mutex> lock(mu);
@@ -1006,17 +997,17 @@ int tune_slice(qd_handle *h)
   cudaEvent_t e0, e1;
   CU(cudaEventCreate(&e0));
   CU(cudaEventCreate(&e1));
-  LineParams p = line_params(h, f32);
+  LineParams p = line_params(h, true);
   float best = 1e30f;
-  for (int cl : {0, 1, 2, 4, SLICE_RF, SLICE_RF2, SLICE_RF4, SLICE_RF4W, SLICE_AX, SLICE_AX2}) {
-    if (!tried(cl)) continue;
+  for (int cl : {0, 1, 2, 4, SLICE_RF, SLICE_RF2, SLICE_RF4, SLICE_RF4W}) {
+    if (rf ? !slice_is_rf(cl) || !built(cl) : cl > 0 && !built(cl)) continue;
     p.cluster = cl;
     bool ok = true;
     for (int it = 0; it < 2 && ok; it++)
-      ok = run_lines(p, f32, h->st) == cudaSuccess;
+      ok = run_lines(p, true, h->st) == cudaSuccess;
     if (ok) ok = cudaEventRecord(e0, h->st) == cudaSuccess;
     for (int it = 0; it < 5 && ok; it++)
-      ok = run_lines(p, f32, h->st) == cudaSuccess;
+      ok = run_lines(p, true, h->st) == cudaSuccess;
     if (ok) ok = cudaEventRecord(e1, h->st) == cudaSuccess;
     if (ok) ok = cudaStreamSynchronize(h->st) == cudaSuccess;
     float ms = 0.f;
@@ -1029,8 +1020,7 @@ int tune_slice(qd_handle *h)
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
-  CU(cudaMemsetAsync(h->d_lpsi, 0, (f32 ? sizeof(float2) : sizeof(double2)) * h->n12 * h->nl *
-                                       h->nruns, h->st));
+  CU(cudaMemsetAsync(h->d_lpsi, 0, sizeof(float2) * h->n12 * h->nl * h->nruns, h->st));
   std::lock_guard<std::mutex> lock(mu);
   chosen[key] = h->slice_cluster;
   return QD_OK;
@@ -1151,7 +1141,7 @@ template <typename R> int issue_lines(qd_handle *h)
   TRY(prof_mark(h, -1));
   CU(run_lines(p, sizeof(R) == 4, h->st));
   g_launches += p.cluster == 0 ? lines_launches_per_step(h->n1, h->n2, h->prec)
-              : p.cluster == SLICE_AX2 ? 2 : 1;
+              : p.cluster == SLICE_AX ? 2 : 1;
   TRY(prof_mark(h, PROF_LINES));
   if (fused_flux) TRY(after_flux_prep(h));
   return QD_OK;
@@ -1252,7 +1242,7 @@ template <typename Real> int propagate(qd_handle *h, int n, size_t flush_bytes =
     return h->d_esum + (long)(t / every - steps0 / every - 1) * R * 3;
   };
   const bool split_ok = h->slice_cluster == 0 || slice_is_rf(h->slice_cluster) ||
-                        slice_is_ax(h->slice_cluster);
+                        h->slice_cluster == SLICE_AX;
   for (int s = 0; s < n; s++) {
     const bool redo = !h->started || (s == 0 && h->last_finalized);
     h->esum_col = redo ? nullptr : slot(h->steps);
@@ -1527,6 +1517,7 @@ int create(const qd_data *runs, int nruns, qd_handle **out)
     }
     TRY(upload(h, dim == 0 ? h->d_tw1_64 : h->d_tw2_64, z.data(), n));
     TRY(upload(h, dim == 0 ? h->d_tw1_32 : h->d_tw2_32, f.data(), n));
+    if (!f64) TRY(upload(h, dim == 0 ? h->d_ts1 : h->d_ts2, axis_f32_twiddles(n, f).data(), n));
   }
   for (int t = 0; t < h->nsets; t++) {
     const size_t o = t * sstride;
@@ -1537,7 +1528,7 @@ int create(const qd_data *runs, int nruns, qd_handle **out)
   }
   if (f64) {
     TRY(h->alloc(h->d_expV, npt * npot));
-    if (axis_f64(h, false)) {
+    if (axis_f64(h)) {
       TRY(h->alloc(h->d_zr1, (size_t)h->jrows * h->n1));
       TRY(h->alloc(h->d_zr2, (size_t)h->jrows * h->n2));
       TRY(h->alloc(h->d_zk1, h->n1));

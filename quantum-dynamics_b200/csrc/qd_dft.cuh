@@ -1,11 +1,9 @@
-// qd_dft.cuh -- DFTs of up to 20 points in registers, natural order in and out,
-// for float2 and double2.  SGN = -1: exp(-2 pi i n m / N), +1: exp(+...).
+// qd_dft.cuh -- FP64 DFTs of up to 20 points in registers, natural order in and
+// out.  SGN = -1: exp(-2 pi i n m / N), +1: exp(+...).
 //
 // Composite sizes are P x Q: n = p + P q, Q-point DFTs over q, twiddles
 // W_N^{p c}, P-point DFTs over p, X[c + Q d].  Constants come from
-// cos_turn() at compile time; the float forms multiply by value + residual (a
-// rounded constant alone would scale every output by a fixed 1 - O(1e-8), a
-// norm drift over a long propagation).
+// cos_turn() at compile time.
 #pragma once
 #include "qd_device.cuh"
 
@@ -35,13 +33,6 @@ template <long N, long D> __device__ __forceinline__ double2 kscale(double2 z)
   constexpr double c = cos_turn(N, D);
   return make_double2(c * z.x, c * z.y);
 }
-template <long N, long D> __device__ __forceinline__ float2 kscale(float2 z)
-{
-  constexpr double c = cos_turn(N, D);
-  constexpr float hi = (float)c, lo = (float)(c - (double)hi);
-  return cscale2(z, hi, lo);
-}
-
 // z * exp(SGN 2 pi i E / N)
 template <int N, int E, int SGN, typename C> __device__ __forceinline__ C twk(C z)
 {

@@ -9,6 +9,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <vector>
 #include "qd_device.cuh"
 
 // Column pass modes
@@ -114,8 +115,9 @@ struct LineParams {
   //   kin = kc1[i] kc2[j] (kscale + kscale_lo),  kc1 = exp(-i T1 dt), kc2 likewise
   const float2 *rc1, *rc2;
   const float2 *kc1, *kc2;
-  // FP64: the same factors in FP64 (k_axis.cuh); rot and kin are null then
+  // FP64: the same factors in FP64 (k_axis_f64.cu); rot and kin are null then
   const double2 *zr1, *zr2, *zk1, *zk2;
+  const float2 *ts1, *ts2; // second-group twiddles of n1, n2 (k_axis_f32.cu)
   float kscale, kscale_lo; // FP32: 1/(n1 n2) = kscale + kscale_lo
   const void *tw1, *tw2;   // complex<R> root tables of n1, n2
   FftPlan pl1, pl2;
@@ -257,19 +259,12 @@ constexpr int SLICE_RF = 8;    // LineParams::cluster value of the register-FFT 
 constexpr int SLICE_RF2 = 9;   // the same on a 2-CTA cluster per slice
 constexpr int SLICE_RF4 = 10;  // the same on a 4-CTA cluster per slice
 constexpr int SLICE_RF4W = 11; // the 4-CTA form with 16 x 16 row transforms
-constexpr int SLICE_AX = 12;   // run-time register-FFT kernel (k_axis.cuh), one CTA per slice
-constexpr int SLICE_AX2 = 13;  // the same as a row and a column launch
-inline bool slice_is_ax(int cluster) { return cluster == SLICE_AX || cluster == SLICE_AX2; }
-// factors, row layout and block sizes of a grid for k_axis.cuh (elem: bytes of a complex value)
-struct AxisPlan {
-  int A1, B1, A2, B2;      // n1 = A1 B1, n2 = A2 B2
-  int bs, RS;              // row array: block and row stride
-  int hr, nrb, tc, ncb;    // rows per CTA and blocks, columns per CTA and blocks (split forms)
-  unsigned mA1, mB1, mQ;   // e / A1, e / B1, e / (columns of a CTA) = umulhi(e, m)
-  int max_radix;
-};
-bool axis_plan(int n1, int n2, int elem, bool fused, AxisPlan &out);
-int axis_threads(int cluster);
+constexpr int SLICE_AX = 12;   // run-time register-FFT kernels, a row and a column launch
+// the grids k_axis_f32.cu and k_axis_f64.cu take, and their launches
+bool axis_f32_ok(int n1, int n2);
+bool axis_f64_ok(int n1, int n2);
+int axis_threads();
+std::vector<float2> axis_f32_twiddles(int n, const std::vector<float2> &roots);
 cudaError_t launch_axis_f32(const LineParams &p, cudaStream_t s);
 cudaError_t launch_axis_f64(const LineParams &p, cudaStream_t s);
 inline bool slice_is_rf(int cluster)
@@ -280,7 +275,7 @@ inline bool slice_is_rf(int cluster)
 inline int slice_ctas(int cluster)           // CTAs per slice
 {
   return cluster == SLICE_RF ? 1 : cluster == SLICE_RF2 ? 2
-       : cluster == SLICE_RF4 || cluster == SLICE_RF4W ? 4 : slice_is_ax(cluster) ? 1 : cluster;
+       : cluster == SLICE_RF4 || cluster == SLICE_RF4W ? 4 : cluster == SLICE_AX ? 1 : cluster;
 }
 int slice_cluster_ok(int n1, int n2, int cluster);
 int slice_rf_threads(int n1, int n2, int cl); // threads per CTA, 0 if the shape is not built
