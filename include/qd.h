@@ -236,7 +236,7 @@ int qd_kernel_times(qd_handle *h, double *ms_out, int32_t n, int32_t *n_written)
  * form with 16 x 16 row transforms, 12 the run-time register-FFT kernels;
  * 0 for the FP64 form), out[1] = 1 if the
  * column pass runs on the tensor cores, out[2] = the flux-accumulation GEMM
- * tile variant (0-3), out[3] = 1 if full 250-step chunks of flux history are
+ * tile variant (0, 1), out[3] = 1 if full 250-step chunks of flux history are
  * accumulated in the chirp-z form (energies on a uniform grid). */
 int qd_kernel_choice(qd_handle *h, int32_t out[4]);
 

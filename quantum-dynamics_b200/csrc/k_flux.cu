@@ -38,52 +38,69 @@ __global__ void __launch_bounds__(256) k_flux_phase(AccumParams p)
 }
 
 // phi[e][q] += sum_t phase[e][t] psi_s[t][q] (and dphi with the gradient), a
-// complex FP64 GEMM per run.  CTA tile: GE energies x GQ surface points x
-// {psi_s, d psi_s}; each thread owns 4 energies x 4 columns (2 points x 2
-// fields) in registers, GE / 4 x 16 threads.  KT steps of phases and history
-// are staged in shared memory by asynchronous copies into two buffers, so the
-// next KT steps load while the current ones are multiplied; the history is
-// read from HBM once per energy tile.  The variant (GE, KT) is picked per
-// shape by the autotuner.
+// complex FP64 GEMM per run on the FP64 tensor cores (mma.sync m16n8k8 .f64).
+// One 16-row operand holds eight energies, rows 0-7 the real and 8-15 the
+// imaginary part of the result, and the eight contraction slots are four steps
+// times (real, imaginary): of Phi = phase[e][t] a thread needs (Re, Im, -Im, Re)
+// and of psi (Re, Im), one 16-byte load each from the arrays as they are, and no
+// product is wasted.  CTA tile: 16 MG energies x GQ points x {psi_s, d psi_s}; a
+// warp has 8 MG energies and eight points of both fields, so phi and dphi of a
+// point meet in one thread for P(E).  KT steps are staged by asynchronous copies
+// into two buffers.  Strides: a Phi row KT + 4 and a psi row 2 GQ + 2 complex
+// values, so that 16-byte accesses of a quarter-warp touch every bank group once.
+// Bound: FP64 tensor rate (37 TFLOP/s measured) and, in short chunks, reading and
+// writing phi and dphi (32-byte accesses).  250 steps of 241 energies on 8192
+// points (7.9 GFLOP, 250 MB): 398 us on plain FMAs, 278 so; of 150 energies on 3
+// runs of 5400 points: 505, 377.  MG = 4 reads the history less often, MG = 2
+// wastes less of a last energy tile and fills the SMs better (the tuner times
+// both: 278 and 298, 425 and 377).  KT = 32: 311, 366.
 constexpr int GQ = 32;
+constexpr int KT = 16;
+constexpr int PH_LD = KT + 4, PS_LD = 2 * GQ + 2;
 
 __device__ __forceinline__ void cp16(void *dst, const void *src, bool valid)
 {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   const int n = valid ? 16 : 0;                 // 0: fill the 16 bytes with zeros
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" :: "r"(d), "l"(src), "r"(n)
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(d), "l"(src), "r"(n)
                : "memory");
 }
 
-template <int GE, int KT>
-__global__ void __launch_bounds__(GE * 4) k_flux_gemm(AccumParams p)
+template <int MG> constexpr size_t gemm_smem()
+{ return 2 * sizeof(double2) * ((size_t)16 * MG * PH_LD + KT * PS_LD); }
+
+template <int MG>
+__global__ void __launch_bounds__(256, 2) k_flux_gemm(AccumParams p)
 {
-  constexpr int NT = GE * 4;                    // threads: GE / 4 energy groups x 16
-  __shared__ double2 As[2][GE][KT + 1];         // phases (padded rows)
-  __shared__ double2 Bs[2][KT][2 * GQ];         // cols 0..GQ-1 psi_s, GQ..2GQ-1 gradient
-  const int tid = threadIdx.x;
-  const int te = tid >> 4, tc = tid & 15;       // GE/4 energy groups x 16 column groups
+  constexpr int GE = 16 * MG;
+  extern __shared__ double2 fg[];
+  double2 *Ph = fg, *Ps = fg + 2 * GE * PH_LD;  // [2][GE][PH_LD], [2][KT][PS_LD]
+  __shared__ double red[4][GE];                 // P(E) shares of the four point groups
+  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int we = (tid >> 5) >> 2, wq = (tid >> 5) & 3;   // warp: energies 8 MG we.., points 8 wq..
   const int e0 = blockIdx.x * GE, q0 = blockIdx.y * GQ, run = blockIdx.z;
   const double2 *ph = p.phase + ((size_t)run * p.ne) * TMAX;
   auto stage = [&](int buf, int t0) {
-    for (int x = tid; x < GE * KT; x += NT) {
-      const int e = x / KT, t = x % KT;
-      const bool ok = e0 + e < p.ne && t0 + t < p.nt;
-      cp16(&As[buf][e][t], ok ? ph + (size_t)(e0 + e) * TMAX + t0 + t : ph, ok);
+    for (int x = tid; x < GE * KT; x += 256) {
+      const int e = x / KT, s = x % KT;
+      const bool ok = e0 + e < p.ne && t0 + s < p.nt;
+      cp16(Ph + (buf * GE + e) * PH_LD + s, ok ? ph + (size_t)(e0 + e) * TMAX + t0 + s : ph, ok);
     }
-    for (int x = tid; x < KT * 2 * GQ; x += NT) {
-      const int t = x / (2 * GQ), c = x % (2 * GQ), q = q0 + (c % GQ);
-      const bool ok = t0 + t < p.nt && q < p.nq;
-      const size_t o = ok ? ((size_t)(t0 + t) * p.nruns + run) * p.nq + q : 0;
-      cp16(&Bs[buf][t][c], (c < GQ ? p.ring_psi : p.ring_g) + o, ok);
+    for (int x = tid; x < KT * 2 * GQ; x += 256) {
+      const int s = x / (2 * GQ), c = x % (2 * GQ), q = q0 + (c % GQ);
+      const bool ok = t0 + s < p.nt && q < p.nq;
+      const size_t o = ok ? ((size_t)(t0 + s) * p.nruns + run) * p.nq + q : 0;
+      cp16(Ps + (buf * KT + s) * PS_LD + c, (c < GQ ? p.ring_psi : p.ring_g) + o, ok);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  double2 acc[4][4];
+  double acc[MG][2][4];                         // energies 8 m + g, fields, (Re, Re, Im, Im) of 2 points
 #pragma unroll
-  for (int i = 0; i < 4; i++)
+  for (int m = 0; m < MG; m++)
 #pragma unroll
-    for (int j = 0; j < 4; j++) acc[i][j] = make_double2(0.0, 0.0);
+    for (int f = 0; f < 2; f++)
+#pragma unroll
+      for (int i = 0; i < 4; i++) acc[m][f][i] = 0.0;
   const int nchunk = (p.nt + KT - 1) / KT;
   stage(0, 0);
   for (int ch = 0; ch < nchunk; ch++) {
@@ -95,84 +112,83 @@ __global__ void __launch_bounds__(GE * 4) k_flux_gemm(AccumParams p)
       asm volatile("cp.async.wait_group 0;" ::: "memory");
     }
     __syncthreads();
-#pragma unroll 2
-    for (int k = 0; k < KT; k++) {             // rows past nt were zero-filled
-      double2 a[4], b[4];
+    const double2 *pa = Ph + (buf * GE + 8 * MG * we + g) * PH_LD + t;
+    const double2 *pb = Ps + (buf * KT + t) * PS_LD + 8 * wq + g;
 #pragma unroll
-      for (int i = 0; i < 4; i++) a[i] = As[buf][te + (GE / 4) * i][k];
+    for (int k = 0; k < KT; k += 4) {           // steps past nt were zero-filled
+      double2 a[MG], b[2];
 #pragma unroll
-      for (int j = 0; j < 4; j++) b[j] = Bs[buf][k][tc + 16 * j];
+      for (int m = 0; m < MG; m++) a[m] = pa[8 * m * PH_LD + k];
+      b[0] = pb[k * PS_LD];
+      b[1] = pb[k * PS_LD + GQ];
 #pragma unroll
-      for (int i = 0; i < 4; i++)
+      for (int m = 0; m < MG; m++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          acc[i][j].x = fma(a[i].x, b[j].x, fma(-a[i].y, b[j].y, acc[i][j].x));
-          acc[i][j].y = fma(a[i].x, b[j].y, fma(a[i].y, b[j].x, acc[i][j].y));
-        }
+        for (int f = 0; f < 2; f++)
+          asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3}, {%4,%5,%6,%7}, "
+              "{%8,%9}, {%0,%1,%2,%3};"
+              : "+d"(acc[m][f][0]), "+d"(acc[m][f][1]), "+d"(acc[m][f][2]), "+d"(acc[m][f][3])
+              : "d"(a[m].x), "d"(a[m].y), "d"(-a[m].y), "d"(a[m].x), "d"(b[f].x), "d"(b[f].y));
     }
     __syncthreads();                            // buffer free for the stage after next
   }
-  // phi += acc, two energy rows at a time: their eight loads are all issued
-  // before any of their stores (a store between two loads would make each
-  // load wait for the one before, since phi and dphi may alias as far as the
-  // compiler knows)
-  auto at = [&](int i, int j) -> double2 * {
-    const int e = e0 + te + (GE / 4) * i, c = tc + 16 * j, q = q0 + (c % GQ);
-    if (e >= p.ne || q >= p.nq) return nullptr;
-    return (c < GQ ? p.fai : p.dfai) + ((size_t)run * p.ne + e) * p.nq + q;
-  };
-  // with crp_part: this tile's share of P(E), the sum over its points of
-  // w_k Im(conj(phi) dphi) of the updated values (columns j and j + 2 of a
-  // thread are phi and dphi of one point; entries past n_E or past the
-  // surface are zero), formed as each energy row pair is written and reduced
-  // over the 16 column groups of each row at the end.  A tile of GQ points
-  // spans at most two theta rows when n1 >= GQ.
+  // phi += acc by 32-byte accesses, two energy groups at a time: their loads are
+  // all issued before any of their stores.
+  // With crp_part: this tile's share of P(E), the sum over its points of
+  // w_k Im(conj(phi) dphi) of the updated values.
   const bool want_pe = p.crp_part != nullptr;
-  double wq[2] = {0.0, 0.0};
-  if (want_pe) {
-    const int k0 = q0 / p.n1;
+  const int q = q0 + 8 * wq + 2 * t;            // this thread's points q, q + 1
+  double wt[2] = {0.0, 0.0};
+  if (want_pe)
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-      const int q = q0 + tc + 16 * j;
-      const int k = p.n1 >= GQ ? (q - k0 * p.n1 >= p.n1 ? k0 + 1 : k0) : q / p.n1;
-      wq[j] = q < p.nq ? __ldg(p.w + k) : 0.0;
-    }
-  }
-  double pe[4];
+    for (int i = 0; i < 2; i++)
+      if (q + i < p.nq) wt[i] = __ldg(p.w + (q + i) / p.n1);
 #pragma unroll
-  for (int h = 0; h < 4; h += 2) {
+  for (int h = 0; h < MG; h += 2) {
+    double z[2][2][4];                          // two groups, fields, (Re, Im) of q and of q + 1
+    auto at = [&](int m, int f) -> double2 * {  // 32-byte aligned: q and n_q = n_theta n1 are even
+      const int e = e0 + 8 * (MG * we + h + m) + g;
+      if (e >= p.ne || q >= p.nq) return nullptr;
+      return (f ? p.dfai : p.fai) + ((size_t)run * p.ne + e) * p.nq + q;
+    };
 #pragma unroll
-    for (int i = h; i < h + 2; i++)
+    for (int m = 0; m < 2; m++)
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const double2 *src = at(i, j);
-        if (src) {
-          const double2 f = *src;
-          acc[i][j].x += f.x;
-          acc[i][j].y += f.y;
+      for (int f = 0; f < 2; f++) {
+        z[m][f][0] = z[m][f][1] = z[m][f][2] = z[m][f][3] = 0.0;
+        if (const double2 *src = at(m, f))
+          asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];"
+                       : "=d"(z[m][f][0]), "=d"(z[m][f][1]), "=d"(z[m][f][2]), "=d"(z[m][f][3])
+                       : "l"(src) : "memory");
+      }
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+#pragma unroll
+      for (int f = 0; f < 2; f++) {
+#pragma unroll
+        for (int i = 0; i < 2; i++) {
+          z[m][f][2 * i] += acc[h + m][f][i];
+          z[m][f][2 * i + 1] += acc[h + m][f][2 + i];
         }
+        if (double2 *dst = at(m, f))
+          asm volatile("st.global.v4.f64 [%0], {%1,%2,%3,%4};"
+                       :: "l"(dst), "d"(z[m][f][0]), "d"(z[m][f][1]), "d"(z[m][f][2]), "d"(z[m][f][3])
+                       : "memory");
       }
-#pragma unroll
-    for (int i = h; i < h + 2; i++) {
-#pragma unroll
-      for (int j = 0; j < 4; j++) {
-        double2 *dst = at(i, j);
-        if (dst) *dst = acc[i][j];
+      if (want_pe) {                            // over the warp's eight points
+        double pe = wt[0] * (z[m][0][0] * z[m][1][1] - z[m][0][1] * z[m][1][0]) +
+                    wt[1] * (z[m][0][2] * z[m][1][3] - z[m][0][3] * z[m][1][2]);
+        pe += __shfl_xor_sync(0xffffffffu, pe, 1);
+        pe += __shfl_xor_sync(0xffffffffu, pe, 2);
+        if (t == 0) red[wq][8 * (MG * we + h + m) + g] = pe;
       }
-      pe[i] = wq[0] * (acc[i][0].x * acc[i][2].y - acc[i][0].y * acc[i][2].x) +
-              wq[1] * (acc[i][1].x * acc[i][3].y - acc[i][1].y * acc[i][3].x);
     }
   }
   if (want_pe) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      double sum = pe[i];
-#pragma unroll
-      for (int o = 8; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      const int e = e0 + te + (GE / 4) * i;
-      if (tc == 0 && e < p.ne)
-        p.crp_part[((size_t)run * p.ne + e) * gridDim.y + blockIdx.y] = sum;
-    }
+    __syncthreads();
+    if (tid < GE && e0 + tid < p.ne)
+      p.crp_part[((size_t)run * p.ne + e0 + tid) * gridDim.y + blockIdx.y] =
+          red[0][tid] + red[1][tid] + red[2][tid] + red[3][tid];
   }
 }
 
@@ -390,10 +406,15 @@ __global__ void __launch_bounds__(256) k_crp_parts(CrpParams p, const double *pa
   if (threadIdx.x == 0) p.crp[b] = s / p.eta_sq[b] * p.dr1_mu2;
 }
 
-template <int GE, int KT> void launch_gemm(const AccumParams &p, cudaStream_t s)
+template <int MG> cudaError_t launch_gemm(const AccumParams &p, cudaStream_t s)
 {
+  constexpr int GE = 16 * MG;
+  cudaError_t e = cudaFuncSetAttribute(k_flux_gemm<MG>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)gemm_smem<MG>());
+  if (e != cudaSuccess) return e;
   dim3 grid((p.ne + GE - 1) / GE, (p.nq + GQ - 1) / GQ, p.nruns);
-  k_flux_gemm<GE, KT><<<grid, GE * 4, 0, s>>>(p);
+  k_flux_gemm<MG><<<grid, 256, gemm_smem<MG>(), s>>>(p);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -408,7 +429,7 @@ cudaError_t launch_flux_prep(const FluxParams &p, cudaStream_t s)
 template cudaError_t launch_flux_prep<float>(const FluxParams &, cudaStream_t);
 template cudaError_t launch_flux_prep<double>(const FluxParams &, cudaStream_t);
 
-int flux_variants() { return 4; }
+int flux_variants() { return 2; }
 
 bool flux_accum_is_czt(const AccumParams &p)
 {
@@ -440,13 +461,7 @@ cudaError_t launch_flux_accum(const AccumParams &p, cudaStream_t s)
   }
   const int n = p.nruns * p.ne * p.nt;
   k_flux_phase<<<(n + 255) / 256 < 4096 ? (n + 255) / 256 : 4096, 256, 0, s>>>(p);
-  switch (p.variant) {   // (energies per CTA, steps per staged chunk)
-    case 1: launch_gemm<64, 5>(p, s); break;
-    case 2: launch_gemm<32, 10>(p, s); break;
-    case 3: launch_gemm<32, 15>(p, s); break;
-    default: launch_gemm<64, 10>(p, s); break;
-  }
-  return cudaGetLastError();
+  return p.variant == 1 ? launch_gemm<2>(p, s) : launch_gemm<4>(p, s);
 }
 
 cudaError_t launch_crp(const CrpParams &p, cudaStream_t s)
