@@ -452,9 +452,6 @@ bool plan(int n1, int n2, Plan &out)
   Plan p{};
   if (!axis(n1, p.x1) || !axis(n2, p.x2)) return false;
   row_layout(p.x1, p.bs, p.RS, p.RY);
-  p.hr = std::max(1, std::min(n2, 2048 / n1));
-  p.nrb = (n2 + p.hr - 1) / p.hr;
-  p.hr = (n2 + p.nrb - 1) / p.nrb;
   p.ncb = (n1 + TCOLS - 1) / TCOLS;
   plans[{n1, n2}] = p;
   out = p;
@@ -470,6 +467,18 @@ bool axis_f32_ok(int n1, int n2)
 }
 
 int axis_threads() { return NT; }
+
+// Rows per CTA of the row launches (both precisions): about 2048 elements, and
+// fewer where that leaves less than two CTAs per SM (FP64 step: 64 x 64 x 39
+// 26 -> 22 us, 100 x 54 x 29 26 -> 21 us; four per SM cost as much as they gain)
+int axis_rows(int n1, int n2, int slices)
+{
+  const long fill = (long)n2 * slices / 296;
+  const int most = std::max(1, std::min(n2, 2048 / n1));
+  const int hr = (int)std::max(1L, std::min((long)most, fill));
+  const int blocks = (n2 + hr - 1) / hr;
+  return (n2 + blocks - 1) / blocks;
+}
 
 // second-group twiddles of a size from its n complex64 roots, laid out [entry][c]
 // (consecutive items read consecutive values): entries q - 1 (0 < q < r3) are
@@ -492,6 +501,8 @@ cudaError_t launch_axis_f32(const LineParams &p, cudaStream_t s)
 {
   Plan ax;
   if (!plan(p.n1, p.n2, ax)) return cudaErrorInvalidValue;
+  ax.hr = axis_rows(p.n1, p.n2, p.nruns * p.nl);
+  ax.nrb = (p.n2 + ax.hr - 1) / ax.hr;
   cudaError_t e = launch_one<ROWS>(p, ax, s);
   return e != cudaSuccess ? e : launch_one<COLS>(p, ax, s);
 }

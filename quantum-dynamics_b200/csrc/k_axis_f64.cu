@@ -369,9 +369,6 @@ bool plan(int n1, int n2, Plan &out)
   if (!factor(n1, x.A1, x.B1) || !factor(n2, x.A2, x.B2)) return false;
   x.max_radix = std::max(x.A1, x.A2);
   row_layout(x.A1, x.B1, sizeof(double2), x.bs, x.RS);
-  x.hr = std::max(1, std::min(n2, 2048 / n1));
-  x.nrb = (n2 + x.hr - 1) / x.hr;
-  x.hr = (n2 + x.nrb - 1) / x.nrb;
   x.tc = 8;                                  // whole 128-byte segments
   x.ncb = (n1 + x.tc - 1) / x.tc;
   x.mA1 = magic(x.A1);
@@ -394,5 +391,7 @@ cudaError_t launch_axis_f64(const LineParams &p, cudaStream_t s)
 {
   Plan ax;
   if (!plan(p.n1, p.n2, ax)) return cudaErrorInvalidValue;
+  ax.hr = axis_rows(p.n1, p.n2, p.nruns * p.nl);
+  ax.nrb = (p.n2 + ax.hr - 1) / ax.hr;
   return ax.max_radix > 16 ? launch_both<20>(p, ax, s) : launch_both<16>(p, ax, s);
 }

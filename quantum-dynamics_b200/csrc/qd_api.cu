@@ -600,7 +600,6 @@ struct qd_handle {
   double2 *d_expV = nullptr, *d_rot = nullptr, *d_kin = nullptr;
   double2 *d_zr1 = nullptr, *d_zr2 = nullptr, *d_zk1 = nullptr, *d_zk2 = nullptr;
   float2 *d_expV32 = nullptr;
-  float2 *d_ts1 = nullptr, *d_ts2 = nullptr;
   float2 *d_rc1 = nullptr, *d_rc2 = nullptr, *d_kc1 = nullptr, *d_kc2 = nullptr;
   int slice_cluster = 0;          // l-space kernel (LineParams::cluster code)
   int flux_variant = 0;           // flux-accumulation GEMM tile variant (tune_flux)
@@ -920,14 +919,16 @@ LineParams line_params(qd_handle *h, bool f32)
   p.nruns = h->nruns;
   p.rot = h->d_rot; p.kin = h->d_kin;
   p.rc1 = h->d_rc1; p.rc2 = h->d_rc2; p.kc1 = h->d_kc1; p.kc2 = h->d_kc2;
-  p.ts1 = h->d_ts1; p.ts2 = h->d_ts2;
   p.zr1 = h->d_zr1; p.zr2 = h->d_zr2; p.zk1 = h->d_zk1; p.zk2 = h->d_zk2;
   p.cluster = h->slice_cluster;
   const double ks = 1.0 / ((double)h->n1 * h->n2);
   p.kscale = (float)ks;
   p.kscale_lo = (float)(ks - (double)p.kscale);
   if (!f32) { p.tw1 = h->d_tw1_64; p.tw2 = h->d_tw2_64; }
-  else { p.tw1 = h->d_tw1_32; p.tw2 = h->d_tw2_32; }
+  else {
+    p.tw1 = h->d_tw1_32; p.tw2 = h->d_tw2_32;
+    p.ts1 = h->d_tw1_32 + h->n1; p.ts2 = h->d_tw2_32 + h->n2;
+  }
   p.pl1 = h->pl1; p.pl2 = h->pl2;
   p.run_k = h->d_run_k; p.jrows = h->jrows;
   p.T1 = h->d_T1; p.T2 = h->d_T2; p.I1 = h->d_I1; p.I2 = h->d_I2;
@@ -1052,7 +1053,7 @@ template <typename F> float time_launches(qd_handle *h, F launch, int reps = 3)
 // Autotuner of the flux-accumulation GEMM: each tile variant accumulates one
 // full chunk of (still zero) history into the handle's phi_E, which is
 // cleared again afterwards; the fastest is kept per shape for the process.
-// QD_FLUX_VARIANT=0..3 forces a variant.
+// QD_FLUX_VARIANT=0|1 forces a variant.
 int tune_flux(qd_handle *h)
 {
   h->flux_variant = 0;
@@ -1516,8 +1517,10 @@ int create(const qd_data *runs, int nruns, qd_handle **out)
       f[k] = make_float2((float)cosl(a), (float)sinl(a));
     }
     TRY(upload(h, dim == 0 ? h->d_tw1_64 : h->d_tw2_64, z.data(), n));
-    TRY(upload(h, dim == 0 ? h->d_tw1_32 : h->d_tw2_32, f.data(), n));
-    if (!f64) TRY(upload(h, dim == 0 ? h->d_ts1 : h->d_ts2, axis_f32_twiddles(n, f).data(), n));
+    // complex64 roots, then the second-group twiddles of k_axis_f32.cu
+    const std::vector<float2> second = axis_f32_twiddles(n, f);
+    f.insert(f.end(), second.begin(), second.end());
+    TRY(upload(h, dim == 0 ? h->d_tw1_32 : h->d_tw2_32, f.data(), f.size()));
   }
   for (int t = 0; t < h->nsets; t++) {
     const size_t o = t * sstride;

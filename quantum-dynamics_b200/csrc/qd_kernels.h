@@ -264,6 +264,7 @@ constexpr int SLICE_AX = 12;   // run-time register-FFT kernels, a row and a col
 bool axis_f32_ok(int n1, int n2);
 bool axis_f64_ok(int n1, int n2);
 int axis_threads();
+int axis_rows(int n1, int n2, int slices);
 std::vector<float2> axis_f32_twiddles(int n, const std::vector<float2> &roots);
 cudaError_t launch_axis_f32(const LineParams &p, cudaStream_t s);
 cudaError_t launch_axis_f64(const LineParams &p, cudaStream_t s);
