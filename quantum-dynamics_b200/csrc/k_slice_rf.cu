@@ -564,7 +564,8 @@ int slice_rf_threads(int n1, int n2, int cl)
     if (n1 == 128 && n2 == 96) return 256;
     if (n1 == 128 && n2 == 128) return 512;
   } else if (cl == 2) {
-    if (n1 == 128 && n2 == 96) return 256;
+    if (n1 == 64 && n2 == 64) return 256;
+    if (n1 == 128 && n2 == 96) return 256;    // the smaller of its two launches
     if (n1 == 128 && n2 == 128) return 512;
   } else if (cl == 4) {
     if (n1 == 256 && n2 == 192) return 256;   // 128 x 96 and 128 x 128 run faster on CL <= 2
@@ -579,7 +580,13 @@ cudaError_t launch_slice_rf(const LineParams &p, int cl, cudaStream_t s)
     if (p.n1 == 128 && p.n2 == 96) return launch_rf<128, 96, 256, 1>(p, s);
     if (p.n1 == 128 && p.n2 == 128) return launch_rf<128, 128, 512, 1>(p, s);
   } else if (cl == 2) {
-    if (p.n1 == 128 && p.n2 == 96) return launch_rf<128, 96, 256, 2>(p, s);
+    // 64 x 64 x 40: 18.3 us a step on one CTA per slice, 15.0 on two (78 CTAs)
+    if (p.n1 == 64 && p.n2 == 64) return launch_rf<64, 64, 256, 2>(p, s);
+    // one CTA per SM at most: 384 threads instead of 256 (128 x 96 x 64, one run: 18.1 us a
+    // step against 24.1); more CTAs: two of 256 share an SM (two runs: 30.1 against 33.3)
+    if (p.n1 == 128 && p.n2 == 96)
+      return 2 * p.nruns * p.nl <= 148 ? launch_rf<128, 96, 384, 2>(p, s)
+                                       : launch_rf<128, 96, 256, 2>(p, s);
     if (p.n1 == 128 && p.n2 == 128) return launch_rf<128, 128, 512, 2>(p, s);
   } else if (cl == 4) {
     if (p.n1 == 256 && p.n2 == 192) return launch_rf<256, 192, 256, 4>(p, s);
