@@ -17,11 +17,10 @@
 // m16n8k8, one warp per scheduler or more; plain DFMA chains 34).  FP64
 // operands need 8 x 8 values in registers per thread to keep plain FMAs fed
 // from shared memory; with mma the warps of an SM read about 64 B a clock.
-// Tile of 16 columns, not 32: two tiles' buffers (the next one arrives by
-// cp.async while this one is multiplied) fit beside P at 128 x 128, and grids
-// of a few hundred tiles spread over the SMs.  Per launch, against the SIMT
-// kernel: 256 x 192 x 128 (6.4 GFLOP) 835 -> 258 us, 128 x 128 x 64 87 -> 35 us,
-// 64 x 64 x 40 30 -> 13 us (each with 5 us of event and launch time).
+// Tile of 16 columns, not 32: two tiles fit beside P at 128 x 128, one per group
+// of warps, and grids of a few hundred tiles spread over the SMs.  Per launch,
+// against the SIMT kernel: 256 x 192 x 128 (6.4 GFLOP) 835 -> 235 us, 128 x 128 x
+// 64 87 -> 35 us, 64 x 64 x 40 30 -> 14 us (each with 5 us of event and launch time).
 //
 // Shared layouts: a tile is [row][17] complex (17: every 16-byte access of a
 // warp touches the eight bank groups evenly); P is [k][nlp], nlp a multiple of
@@ -57,10 +56,10 @@ __device__ __forceinline__ void cp16(void *dst, const void *src, bool valid)
 
 __host__ __device__ inline int pad8(int n) { return (n + 7) & ~7; }
 __host__ __device__ inline int pad16(int n) { return (n + 15) & ~15; }
-inline size_t dmma_smem(int nth, int nl)
+inline size_t dmma_smem(int nth, int nl, int tiles)
 {
   const size_t rows = pad8(nth) > pad8(nl) ? pad8(nth) : pad8(nl);
-  return sizeof(double) * (size_t)pad8(nth) * pad16(nl) + 2 * sizeof(double2) * rows * LD +
+  return sizeof(double) * (size_t)pad8(nth) * pad16(nl) + tiles * sizeof(double2) * rows * LD +
          sizeof(double) * pad8(nth);
 }
 
@@ -131,37 +130,36 @@ __device__ __forceinline__ void gemm(double (&acc)[MI][NI][4], const double2 *ti
   for (; b < kb; b++) block(b);
 }
 
-// WM x WN warps: warp (wm, wn) takes 16 / WM of the tile's columns and every
-// WN-th group of eight outputs, NI of them
-template <int WM, int WN, int NI, int MODE>
-__global__ void __launch_bounds__(WM * WN * 32, 16 / (WM * WN)) k_column_dmma(ColumnParams p)
+// NG groups of 2 x 4 warps, each with its own tiles and its own barrier: one
+// group's loads, theta-space work and stores overlap the other's products.  In
+// a group warp (wm, wn) takes 8 of the tile's columns and every fourth group of
+// eight outputs, NI of them.
+constexpr int WN = 4, GT = 256;         // warps along the outputs, threads of a group
+template <int NG, int NI, int MODE>
+__global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
 {
-  constexpr int NT = WM * WN * 32, MI = 2 / WM;
+  constexpr int NT = NG * GT;
   extern __shared__ __align__(16) unsigned char smem[];
   const int nthp = pad8(p.nth), nlp = pad16(p.nl), nl8 = pad8(p.nl);
   const int rows = nthp > nl8 ? nthp : nl8;
-  double2 *buf = reinterpret_cast<double2 *>(smem);       // [2][rows][LD]
-  double *P = reinterpret_cast<double *>(buf + 2 * rows * LD);
+  const int tid = threadIdx.x, grp = tid / GT, gtid = tid % GT;
+  const int lane = tid & 31, g = lane >> 2, t = lane & 3;
+  double2 *cur = reinterpret_cast<double2 *>(smem) + grp * rows * LD;   // the group's tile [rows][LD]
+  double *P = reinterpret_cast<double *>(reinterpret_cast<double2 *>(smem) + NG * rows * LD);
   double *w = P + nthp * nlp;
-  const int tid = threadIdx.x, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int wn = (tid >> 5) % WN, c0 = 8 * MI * ((tid >> 5) / WN);   // the warp's first column
+  const int wn = (gtid >> 5) % WN, c0 = 8 * ((gtid >> 5) / WN);   // the warp's first column
   const int n12 = (int)p.n12;
-  const int tiles_per_run = (n12 + TC - 1) / TC;
+  const int tpr = (n12 + TC - 1) / TC;                // tiles per run
+  const int ntiles = tpr * p.nruns;
   const int kgrp = nthp >> 3, lgrp = nl8 >> 3;
   pdl_trigger();
 
-  // tiles blockIdx.x, + gridDim.x, ...: position `at` of the runs' order, tile `in` of that run
-  struct Pos { int at, in; };
-  auto step = [&](Pos x) {
-    x.in += gridDim.x;
-    while (x.in >= tiles_per_run) {
-      x.in -= tiles_per_run;
-      x.at++;
-    }
-    return x;
+  auto group_sync = [&] {
+    if (NG == 1) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" :: "r"(1 + grp), "r"(GT) : "memory");
   };
-  auto run_of = [&](Pos x) { return p.run_order ? p.run_order[x.at] : x.at; };
-  auto load_P = [&](int set) {
+  auto run_at = [&](int at) { return p.run_order ? p.run_order[at] : at; };
+  auto load_P = [&](int set) {                        // by the whole CTA
     const double *src = p.P + set * p.set_stride;
     const int half = nlp >> 1;
     for (int x = tid; x < nthp * half; x += NT) {
@@ -172,15 +170,14 @@ __global__ void __launch_bounds__(WM * WN * 32, 16 / (WM * WN)) k_column_dmma(Co
           make_double2(in && l < p.nl ? __ldg(s) : 0.0, in && l + 1 < p.nl ? __ldg(s + 1) : 0.0);
     }
   };
-  // the l-space tile (MID, TAIL) into buffer b, rows past n_l and columns past the grid zero
-  auto fetch = [&](Pos x, int b) {
-    if (MODE != COL_HEAD && x.at < p.nruns) {
-      const int c = tid % TC, q = x.in * TC + c;
-      const double2 *src = reinterpret_cast<const double2 *>(p.lpsi) +
-                           (long)run_of(x) * p.nl * p.n12;
-      const double2 *s = src + (long)(tid / TC) * n12 + q;
-      double2 *d = buf + (b * rows + tid / TC) * LD + c;
-      for (int l = tid / TC; l < nl8; l += NT / TC, s += (long)(NT / TC) * n12, d += NT / TC * LD) {
+  // the l-space tile (MID, TAIL) into the group's buffer, rows past n_l and columns past the grid zero
+  auto fetch = [&](int tile) {
+    if (MODE != COL_HEAD && tile < ntiles) {
+      const int at = tile / tpr, c = gtid % TC, q = (tile - at * tpr) * TC + c;
+      const double2 *src = reinterpret_cast<const double2 *>(p.lpsi) + (long)run_at(at) * p.nl * p.n12;
+      const double2 *s = src + (long)(gtid / TC) * n12 + q;
+      double2 *d = cur + (gtid / TC) * LD + c;
+      for (int l = gtid / TC; l < nl8; l += GT / TC, s += (long)(GT / TC) * n12, d += GT / TC * LD) {
         const bool ok = l < p.nl && q < n12;
         cp16(d, ok ? s : src, ok);
       }
@@ -189,67 +186,51 @@ __global__ void __launch_bounds__(WM * WN * 32, 16 / (WM * WN)) k_column_dmma(Co
   };
 
   for (int k = tid; k < nthp; k += NT) w[k] = k < p.nth ? p.w[k] : 0.0;
-  Pos pos = {(int)blockIdx.x / tiles_per_run, (int)blockIdx.x % tiles_per_run};
-  int run = run_of(pos), set = p.run_set ? p.run_set[run] : 0;
+  // the CTA's tiles blockIdx.x + i gridDim.x, group i % NG; `at` is their position in the runs' order
+  int at = (int)blockIdx.x / tpr, run = run_at(at), set = p.run_set ? p.run_set[run] : 0;
   load_P(set);
-  pdl_wait();                                       // psi_l: the l-space pass's output
-  fetch(pos, 0);
-  double nsum = 0.0, esum = 0.0;
-  auto flush = [&](int r) {                         // this thread's sums over run r's tiles
-    for (int o = 16; o > 0; o >>= 1) {
-      nsum += __shfl_xor_sync(0xffffffffu, nsum, o);
-      esum += __shfl_xor_sync(0xffffffffu, esum, o);
+  pdl_wait();                                         // psi_l: the l-space pass's output
+  int mine = blockIdx.x + grp * gridDim.x;            // this group's next tile
+  fetch(mine);
+  __syncthreads();                                    // P and w in place
+  const int k0 = 8 * wn + 2 * t;                      // this thread's first angle and first order
+  // all groups walk the runs of the CTA's tiles in step, as they share P
+  for (int tile0 = blockIdx.x; tile0 < ntiles;) {
+    at = tile0 / tpr;
+    run = run_at(at);
+    const int end = (at + 1) * tpr;                   // first tile of the next run
+    const int s = p.run_set ? p.run_set[run] : 0;
+    if (s != set) {                                   // the same for the whole CTA
+      __syncthreads();                                // every read of the old P is done
+      set = s;
+      load_P(set);
+      __syncthreads();
     }
-    if (lane == 0 && p.norm_out) atomicAdd(p.norm_out + r, nsum);
-    if (lane == 0 && p.esum) atomicAdd(p.esum + 3 * r + 2, esum);
-    nsum = esum = 0.0;
-  };
-
-  const int k0 = 8 * wn + 2 * t;                    // this thread's first angle and first order
-  Pos next;
-  for (int it = 0; pos.at < p.nruns; it++, pos = next) {
-    next = step(pos);
-    const int r = run_of(pos);
-    if (r != run) {
-      if (MODE != COL_HEAD) flush(run);
-      run = r;
-      const int s = p.run_set ? p.run_set[run] : 0;
-      if (s != set) {
-        __syncthreads();                            // the previous tile's reads of P are done
-        set = s;
-        load_P(set);
-      }
-    }
-    const int p0 = pos.in * TC;
     const long zoff = (long)run * p.nth * p.n12, voff = (long)run * p.vrun;
-    double2 *cur = buf + (it & 1) * rows * LD;
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();                                // the tile (and P) in place; the other buffer free
-    fetch(next, (it & 1) ^ 1);
+    double nsum = 0.0, esum = 0.0;
+    for (; mine < end; ) {
+      const int p0 = (mine - at * tpr) * TC;
+      mine += NG * gridDim.x;
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      group_sync();                                   // the tile in place
 
-    double acc[MI][NI][4];
-    if (MODE != COL_HEAD) {
-      // exp(-iVdt) of this thread's values, in flight during GEMM1
-      double2 ph[MI][NI][2];
-      if (MODE == COL_MID) {
-#pragma unroll
-        for (int m = 0; m < MI; m++) {
-          const int q = p0 + c0 + 8 * m + g;
+      double acc[1][NI][4];
+      if (MODE != COL_HEAD) {
+        // exp(-iVdt) of this thread's values, in flight during GEMM1
+        const int q = p0 + c0 + g;
+        const bool in = q < n12;
+        double2 ph[NI][2];
+        if (MODE == COL_MID) {
           const double2 *v = p.expV + voff + (long)k0 * n12 + q;
 #pragma unroll
           for (int n = 0; n < NI; n++)
 #pragma unroll
             for (int i = 0; i < 2; i++)
-              if (k0 + 8 * WN * n + i < p.nth && q < n12)
-                ph[m][n][i] = __ldg(v + (long)(8 * WN * n + i) * n12);
+              if (k0 + 8 * WN * n + i < p.nth && in) ph[n][i] = __ldg(v + (long)(8 * WN * n + i) * n12);
         }
-      }
-      gemm<MI, NI, WN, false>(acc, cur + c0, P, nlp, lgrp, kgrp, wn, g, t);
-      __syncthreads();                              // every read of the l-space tile is done
-#pragma unroll
-      for (int m = 0; m < MI; m++) {
-        const int q = p0 + c0 + 8 * m + g;
-        const bool in = q < n12;
+        gemm<1, NI, WN, false>(acc, cur + c0, P, nlp, lgrp, kgrp, wn, g, t);
+        group_sync();                                 // every read of the l-space tile is done
+        if (MODE == COL_TAIL) fetch(mine);
         const int j = in ? q / p.n1 : 0, i1 = in ? q - j * p.n1 : 0;
         const double d = in && p.d1 ? p.d1[i1] * p.d2[j] : 1.0;
         const bool fl = in && p.do_flux && j >= p.surf_j0 && j < p.surf_j0 + p.surf_nrows;
@@ -261,7 +242,7 @@ __global__ void __launch_bounds__(WM * WN * 32, 16 / (WM * WN)) k_column_dmma(Co
 #pragma unroll
           for (int i = 0; i < 2; i++) {
             const int k = k0 + 8 * WN * n + i;
-            double2 v = make_double2(acc[m][n][i], acc[m][n][2 + i]);
+            double2 v = make_double2(acc[0][n][i], acc[0][n][2 + i]);
             if (k < p.nth && in) {
               const double wk = w[k];
               if (p.esum)
@@ -270,71 +251,78 @@ __global__ void __launch_bounds__(WM * WN * 32, 16 / (WM * WN)) k_column_dmma(Co
               if (fl) surf[k * p.n1] = v;
               nsum += wk * (v.x * v.x + v.y * v.y);
               if (MODE == COL_TAIL && p.out_z) p.psi_z[zoff + (long)k * n12 + q] = v;
-              if (MODE == COL_MID) v = cscale(cmul(v, ph[m][n][i]), wk);
+              if (MODE == COL_MID) v = cscale(cmul(v, ph[n][i]), wk);
             } else {
               v = make_double2(0.0, 0.0);
             }
-            if (MODE == COL_MID) cur[k * LD + c0 + 8 * m + g] = v;
+            if (MODE == COL_MID) cur[k * LD + c0 + g] = v;
           }
         }
-      }
-      if (MODE == COL_TAIL) continue;
-    } else {
-      for (int x = tid; x < nthp * TC; x += NT) {
-        const int k = x / TC, c = x % TC, q = p0 + c;
-        const long o = (long)k * n12 + q;
-        double2 z = make_double2(0.0, 0.0);
-        if (k < p.nth && q < n12) {
-          z = p.psi_z[zoff + o];
-          double s, co;
-          sincos(p.dt * p.pot[voff + o], &s, &co);  // exp(-i V dt) = (co, -s)
-          double2 f = make_double2(co, -s);
-          if (p.prestep) {
-            // psi / sqrt(v) * v = psi * sqrt(v), principal branch
-            // (pre_evolution_with_potential_dt_2, timeEvol.C:519-538)
-            double sh, ch;
-            sincos(0.5 * atan2(-s, co), &sh, &ch);
-            f = make_double2(ch, sh);
+        if (MODE == COL_TAIL) continue;
+      } else {
+        for (int x = gtid; x < nthp * TC; x += GT) {
+          const int k = x / TC, c = x % TC, q = p0 + c;
+          const long o = (long)k * n12 + q;
+          double2 z = make_double2(0.0, 0.0);
+          if (k < p.nth && q < n12) {
+            z = p.psi_z[zoff + o];
+            double s, co;
+            sincos(p.dt * p.pot[voff + o], &s, &co);  // exp(-i V dt) = (co, -s)
+            double2 f = make_double2(co, -s);
+            if (p.prestep) {
+              // psi / sqrt(v) * v = psi * sqrt(v), principal branch
+              // (pre_evolution_with_potential_dt_2, timeEvol.C:519-538)
+              double sh, ch;
+              sincos(0.5 * atan2(-s, co), &sh, &ch);
+              f = make_double2(ch, sh);
+            }
+            z = cscale(cmul(z, f), w[k]);
           }
-          z = cscale(cmul(z, f), w[k]);
+          cur[k * LD + c] = z;
         }
-        cur[k * LD + c] = z;
+      }
+      group_sync();                                   // the theta-space tile in place
+      gemm<1, NI, WN, true>(acc, cur + c0, P, nlp, kgrp, lgrp, wn, g, t);
+      group_sync();                                   // every read of it is done
+      fetch(mine);
+      const int q = p0 + c0 + g;
+      if (q < n12) {
+        double2 *dst = reinterpret_cast<double2 *>(p.lpsi) + ((long)run * p.nl + k0) * p.n12 + q;
+#pragma unroll
+        for (int n = 0; n < NI; n++)
+#pragma unroll
+          for (int i = 0; i < 2; i++) {
+            const int l = k0 + 8 * WN * n + i;
+            if (l < p.nl)
+              dst[(long)(8 * WN * n + i) * n12] =
+                  make_double2((l + 0.5) * acc[0][n][i], (l + 0.5) * acc[0][n][2 + i]);
+          }
       }
     }
-    __syncthreads();                                // the theta-space tile in place
-    gemm<MI, NI, WN, true>(acc, cur + c0, P, nlp, kgrp, lgrp, wn, g, t);
-#pragma unroll
-    for (int m = 0; m < MI; m++) {
-      const int q = p0 + c0 + 8 * m + g;
-      if (q >= n12) continue;
-      double2 *dst = reinterpret_cast<double2 *>(p.lpsi) + ((long)run * p.nl + k0) * p.n12 + q;
-#pragma unroll
-      for (int n = 0; n < NI; n++)
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-          const int l = k0 + 8 * WN * n + i;
-          if (l < p.nl)
-            dst[(long)(8 * WN * n + i) * n12] =
-                make_double2((l + 0.5) * acc[m][n][i], (l + 0.5) * acc[m][n][2 + i]);
-        }
+    if (MODE != COL_HEAD) {                           // this thread's sums over the run's tiles
+      for (int o = 16; o > 0; o >>= 1) {
+        nsum += __shfl_xor_sync(0xffffffffu, nsum, o);
+        esum += __shfl_xor_sync(0xffffffffu, esum, o);
+      }
+      if (lane == 0 && p.norm_out) atomicAdd(p.norm_out + run, nsum);
+      if (lane == 0 && p.esum) atomicAdd(p.esum + 3 * run + 2, esum);
     }
+    tile0 += (end - tile0 + gridDim.x - 1) / gridDim.x * gridDim.x;   // the CTA's first tile past this run
   }
-  if (MODE != COL_HEAD) flush(run);
 }
 
-template <int WM, int WN, int NI, int MODE>
+template <int NG, int NI, int MODE>
 cudaError_t launch(const ColumnParams &p, cudaStream_t s)
 {
-  const size_t sm = dmma_smem(p.nth, p.nl);
-  cudaError_t e = cudaFuncSetAttribute(k_column_dmma<WM, WN, NI, MODE>,
+  const size_t sm = dmma_smem(p.nth, p.nl, NG);
+  cudaError_t e = cudaFuncSetAttribute(k_column_dmma<NG, NI, MODE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   const long ntiles = (p.n12 + TC - 1) / TC * p.nruns;
-  const int by_regs = 16 / (WM * WN);
-  const long slots = 148L * (by_regs > 1 && sm <= 113 * 1024 ? by_regs : 1);   // CTAs resident at once
+  const long slots = NG == 1 && sm <= 113 * 1024 ? 2 * 148 : 148;    // CTAs resident at once
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(ntiles < slots ? ntiles : slots));
-  cfg.blockDim = dim3(WM * WN * 32);
+  cfg.blockDim = dim3(NG * GT);
   cfg.dynamicSmemBytes = sm;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -342,17 +330,16 @@ cudaError_t launch(const ColumnParams &p, cudaStream_t s)
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k_column_dmma<WM, WN, NI, MODE>, p);
+  cudaLaunchKernelEx(&cfg, k_column_dmma<NG, NI, MODE>, p);
   return cudaGetLastError();
 }
 
-template <int WM, int WN, int NI>
-cudaError_t launch_mode(const ColumnParams &p, int mode, cudaStream_t s)
+template <int NG, int NI> cudaError_t launch_mode(const ColumnParams &p, int mode, cudaStream_t s)
 {
   switch (mode) {
-    case COL_HEAD: return launch<WM, WN, NI, COL_HEAD>(p, s);
-    case COL_MID: return launch<WM, WN, NI, COL_MID>(p, s);
-    default: return launch<WM, WN, NI, COL_TAIL>(p, s);
+    case COL_HEAD: return launch<NG, NI, COL_HEAD>(p, s);
+    case COL_MID: return launch<NG, NI, COL_MID>(p, s);
+    default: return launch<NG, NI, COL_TAIL>(p, s);
   }
 }
 
@@ -361,14 +348,15 @@ cudaError_t launch_mode(const ColumnParams &p, int mode, cudaStream_t s)
 // P and two tiles in shared memory, and no more than MAXGRP groups on either side
 bool column_dmma_ok(int nth, int nl)
 {
-  return pad8(nth) <= 8 * MAXGRP && pad8(nl) <= 8 * MAXGRP && dmma_smem(nth, nl) <= 227 * 1024;
+  return pad8(nth) <= 8 * MAXGRP && pad8(nl) <= 8 * MAXGRP && dmma_smem(nth, nl, 2) <= 227 * 1024;
 }
 
 cudaError_t launch_column_dmma(const ColumnParams &p, int mode, cudaStream_t s)
 {
-  // 64 angles and orders or fewer: P and two tiles take 68 KB at most, two CTAs
-  // of 8 warps share an SM (128 x 128 x 64: 35.1 us a launch, 39.2 with one CTA of
-  // 16 warps); more: one CTA of 16 warps (256 x 192 x 128: 258 us, 275 with 8)
-  return pad8(p.nth) <= 64 && pad8(p.nl) <= 64 ? launch_mode<2, 4, 2>(p, mode, s)
-                                               : launch_mode<2, 8, 2>(p, mode, s);
+  // 64 angles and orders or fewer: P and a tile take 50 KB at most, two CTAs of one
+  // group share an SM (128 x 128 x 64: 35.1 us a launch; one CTA of two groups 33.2,
+  // but 64 x 64 x 40 14.4 against 13.9); more: one CTA of two groups (256 x 192 x 128:
+  // 235 us; one group of 16 warps with the next tile in a second buffer 256)
+  return pad8(p.nth) <= 64 && pad8(p.nl) <= 64 ? launch_mode<1, 2>(p, mode, s)
+                                               : launch_mode<2, 4>(p, mode, s);
 }
