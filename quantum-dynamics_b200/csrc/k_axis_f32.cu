@@ -25,8 +25,8 @@
 //
 // Bound: the latency of four dependent passes per CTA and two launches for grids
 // of a few hundred slices, then L2 (8 runs of 96 x 96 x 48: 113 MB in 54 us).
-// Per step, best Stockham form -> this: 3 runs of 108 x 90 x 50 99 -> 34 us,
-// 144 x 120 x 64 52 -> 25 us, 256 x 256 x 32 132 -> 48 us.
+// Per step, best Stockham form -> this: 3 runs of 108 x 90 x 50 99 -> 26 us,
+// 144 x 120 x 64 52 -> 25 us, 200 x 180 x 40 93 -> 29 us.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -157,19 +157,24 @@ template <int R3, int R4, int SGN> __device__ __forceinline__ void second(float2
 }
 
 template <int R, int RR> struct Group { static constexpr int r = R, rr = RR; };
-template <typename F> __device__ __forceinline__ void with_group(int code, F f)
+template <bool BIG, typename F> __device__ __forceinline__ void with_group(int code, F f)
 {
-#define QD_GROUP(R, RR) case 16 * R + RR: f(Group<R, RR>()); break;
+#define QD_GROUP(R, RR) case 16 * R + RR: f(Group<R, RR>()); return;
   switch (code) {
     QD_GROUP(2, 1) QD_GROUP(3, 1) QD_GROUP(4, 1) QD_GROUP(5, 1) QD_GROUP(8, 1)
-    QD_GROUP(2, 3) QD_GROUP(2, 5) QD_GROUP(3, 3) QD_GROUP(3, 5) QD_GROUP(4, 3) QD_GROUP(4, 5)
-    QD_GROUP(5, 5) QD_GROUP(8, 2) QD_GROUP(8, 3) QD_GROUP(8, 4)
+    QD_GROUP(2, 3) QD_GROUP(2, 5) QD_GROUP(3, 3) QD_GROUP(3, 5) QD_GROUP(4, 3) QD_GROUP(8, 2)
+  }
+  if constexpr (BIG) switch (code) {
+    QD_GROUP(4, 5) QD_GROUP(5, 5) QD_GROUP(8, 3) QD_GROUP(8, 4)
   }
 #undef QD_GROUP
 }
 
-template <int KIND>
-__global__ void __launch_bounds__(NT, 4) k_axis_f32(LineParams p, Plan ax)
+// BIG: a group of more than 16 points, whose values take more registers; the
+// others run at 64 registers, up to eight CTAs per SM (step of 3 runs of 108 x 90 x 50:
+// 48.4 us at 128 registers for all, 40.4 so; 200 x 180 x 40 46.5 and 39.7)
+template <int KIND, bool BIG>
+__global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan ax)
 {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double red[32];
@@ -227,7 +232,7 @@ __global__ void __launch_bounds__(NT, 4) k_axis_f32(LineParams p, Plan ax)
   const bool en = p.esum != nullptr;
   double e_k = 0.0, e_r = 0.0;
 
-  with_group(x.first, [&](auto gr) {                  // global, D -> X
+  with_group<BIG>(x.first, [&](auto gr) {                  // global, D -> X
     typedef decltype(gr) G;
     constexpr int NB = G::r * G::rr;
     for (int e = tid; e < lines * A; e += NT) {
@@ -245,7 +250,7 @@ __global__ void __launch_bounds__(NT, 4) k_axis_f32(LineParams p, Plan ax)
     }
   });
   __syncthreads();
-  with_group(x.second, [&](auto gr) {                 // X -> K -> Y
+  with_group<BIG>(x.second, [&](auto gr) {                 // X -> K -> Y
     typedef decltype(gr) G;
     constexpr int NA = G::r * G::rr;
     for (int e = tid; e < lines * B; e += NT) {
@@ -272,7 +277,7 @@ __global__ void __launch_bounds__(NT, 4) k_axis_f32(LineParams p, Plan ax)
     }
   });
   __syncthreads();
-  with_group(x.first, [&](auto gr) {                  // Y -> X, inverse
+  with_group<BIG>(x.first, [&](auto gr) {                  // Y -> X, inverse
     typedef decltype(gr) G;
     constexpr int NB = G::r * G::rr;
     for (int e = tid; e < lines * A; e += NT) {
@@ -288,7 +293,7 @@ __global__ void __launch_bounds__(NT, 4) k_axis_f32(LineParams p, Plan ax)
     }
   });
   __syncthreads();
-  with_group(x.second, [&](auto gr) {                 // X, D -> global
+  with_group<BIG>(x.second, [&](auto gr) {                 // X, D -> global
     typedef decltype(gr) G;
     constexpr int NA = G::r * G::rr;
     for (int e = tid; e < lines * B; e += NT) {
@@ -329,11 +334,11 @@ __global__ void __launch_bounds__(NT, 4) k_axis_f32(LineParams p, Plan ax)
   }
 }
 
-template <int KIND> cudaError_t launch_one(const LineParams &p, const Plan &ax, cudaStream_t s)
+template <int KIND, bool BIG> cudaError_t launch_one(const LineParams &p, const Plan &ax, cudaStream_t s)
 {
   const size_t sm = sizeof(float2) * (KIND == ROWS ? (size_t)ax.hr * (ax.RS + ax.RY) + 3 * p.n1
                                                    : 2 * (size_t)p.n2 * TCOLS + 3 * p.n2);
-  cudaError_t e = cudaFuncSetAttribute(k_axis_f32<KIND>,
+  cudaError_t e = cudaFuncSetAttribute(k_axis_f32<KIND, BIG>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
@@ -347,7 +352,7 @@ template <int KIND> cudaError_t launch_one(const LineParams &p, const Plan &ax, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = pdl_enabled() ? 1 : 0;
-  cudaLaunchKernelEx(&cfg, k_axis_f32<KIND>, p, ax);
+  cudaLaunchKernelEx(&cfg, k_axis_f32<KIND, BIG>, p, ax);
   return cudaGetLastError();
 }
 
@@ -503,6 +508,8 @@ cudaError_t launch_axis_f32(const LineParams &p, cudaStream_t s)
   if (!plan(p.n1, p.n2, ax)) return cudaErrorInvalidValue;
   ax.hr = axis_rows(p.n1, p.n2, p.nruns * p.nl);
   ax.nrb = (p.n2 + ax.hr - 1) / ax.hr;
-  cudaError_t e = launch_one<ROWS>(p, ax, s);
-  return e != cudaSuccess ? e : launch_one<COLS>(p, ax, s);
+  const bool big1 = std::max(ax.x1.A, ax.x1.B) > 16, big2 = std::max(ax.x2.A, ax.x2.B) > 16;
+  const cudaError_t e = big1 ? launch_one<ROWS, true>(p, ax, s) : launch_one<ROWS, false>(p, ax, s);
+  if (e != cudaSuccess) return e;
+  return big2 ? launch_one<COLS, true>(p, ax, s) : launch_one<COLS, false>(p, ax, s);
 }

@@ -8,8 +8,8 @@
 //     [D1 IFFT_R K1 FFT_R D1] (each row)  x  [D2 IFFT_r K2 FFT_r D2] (each column),
 // and a length N = A B transform is a B-point and an A-point DFT in registers.
 // Here A and B are run-time values, each pass a switch over the radices built
-// (4 to 16, and 18 and 20 in a second kernel with more registers), so one
-// kernel takes every grid of the form.  Two launches a step, a CTA per block of
+// (4 to 10, to 16 and to 20 in kernels of their own, with the registers that
+// takes), so every grid of the form is taken.  Two launches a step, a CTA per block of
 // rows and per block of columns (about 2048 elements, several CTAs to an SM):
 // a slice in complex128 rarely fits one SM's shared memory, and where it does a
 // CTA per slice was slower (64 x 64 x 39: 18.3 us against 15.0, 96 x 96 x 48: 29
@@ -40,32 +40,29 @@ struct Plan {
   int bs, RS;              // row array: block and row stride
   int hr, nrb, tc, ncb;    // rows per CTA and blocks, columns per CTA and blocks
   unsigned mA1, mB1, mQ;   // e / A1, e / B1, e / tc = umulhi(e, m)
-  int max_radix;
 };
 
 template <int N> struct Radix { static constexpr int value = N; };
 template <int MAXR, typename F> __device__ __forceinline__ void with_radix(int r, F f)
 {
+#define QD_RADIX(N) case N: f(Radix<N>()); return;
   switch (r) {
-    case 4: f(Radix<4>()); break;
-    case 5: f(Radix<5>()); break;
-    case 6: f(Radix<6>()); break;
-    case 8: f(Radix<8>()); break;
-    case 9: f(Radix<9>()); break;
-    case 10: f(Radix<10>()); break;
-    case 12: f(Radix<12>()); break;
-    case 15: f(Radix<15>()); break;
-    case 16: f(Radix<16>()); break;
-    default:
-      if constexpr (MAXR > 16) {
-        if (r == 18) f(Radix<18>());
-        else if (r == 20) f(Radix<20>());
-      }
+    QD_RADIX(4) QD_RADIX(5) QD_RADIX(6) QD_RADIX(8) QD_RADIX(9) QD_RADIX(10)
   }
+  if constexpr (MAXR > 10) switch (r) {
+    QD_RADIX(12) QD_RADIX(15) QD_RADIX(16)
+  }
+  if constexpr (MAXR > 16) switch (r) {
+    QD_RADIX(18) QD_RADIX(20)
+  }
+#undef QD_RADIX
 }
 
+// kernels by the larger radix of their dimension, as its values take the
+// registers (step of 200 x 180 x 40 82 -> 76 us, of 3 runs of 108 x 90 x 50 79 -> 76,
+// against one kernel for both dimensions and all radices up to 16)
 template <int KIND, int MAXR>
-__global__ void __launch_bounds__(NT, MAXR > 16 ? 2 : 4) k_axis_f64(LineParams p, Plan ax)
+__global__ void __launch_bounds__(NT, MAXR > 16 ? 2 : MAXR > 10 ? 4 : 5) k_axis_f64(LineParams p, Plan ax)
 {
   typedef double2 C;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -295,10 +292,11 @@ cudaError_t launch_one(const LineParams &p, const Plan &ax, cudaStream_t s)
   return cudaGetLastError();
 }
 
-template <int MAXR> cudaError_t launch_both(const LineParams &p, const Plan &ax, cudaStream_t s)
+template <int KIND> cudaError_t launch_kind(const LineParams &p, const Plan &ax, cudaStream_t s)
 {
-  cudaError_t e = launch_one<ROWS, MAXR>(p, ax, s);
-  return e != cudaSuccess ? e : launch_one<COLS, MAXR>(p, ax, s);
+  const int r = KIND == ROWS ? ax.A1 : ax.A2;            // the larger radix
+  return r > 16 ? launch_one<KIND, 20>(p, ax, s) : r > 10 ? launch_one<KIND, 16>(p, ax, s)
+                                                          : launch_one<KIND, 10>(p, ax, s);
 }
 
 // n = A B with both radices built, the larger as small as it goes, A >= B (the
@@ -367,7 +365,6 @@ bool plan(int n1, int n2, Plan &out)
   }
   Plan x{};
   if (!factor(n1, x.A1, x.B1) || !factor(n2, x.A2, x.B2)) return false;
-  x.max_radix = std::max(x.A1, x.A2);
   row_layout(x.A1, x.B1, sizeof(double2), x.bs, x.RS);
   x.tc = 8;                                  // whole 128-byte segments
   x.ncb = (n1 + x.tc - 1) / x.tc;
@@ -393,5 +390,6 @@ cudaError_t launch_axis_f64(const LineParams &p, cudaStream_t s)
   if (!plan(p.n1, p.n2, ax)) return cudaErrorInvalidValue;
   ax.hr = axis_rows(p.n1, p.n2, p.nruns * p.nl);
   ax.nrb = (p.n2 + ax.hr - 1) / ax.hr;
-  return ax.max_radix > 16 ? launch_both<20>(p, ax, s) : launch_both<16>(p, ax, s);
+  const cudaError_t e = launch_kind<ROWS>(p, ax, s);
+  return e != cudaSuccess ? e : launch_kind<COLS>(p, ax, s);
 }
