@@ -4,17 +4,18 @@
 //     psi_l <- Rot(dt/2) IFFT2 [exp(-i(T1+T2)dt)/(n1 n2)] FFT2 Rot(dt/2) psi_l
 // (evolution_dt, timeEvol.C:625-635; tables timeEvol.C:465-517).
 //
-// The separable phases make the slice operator a row operator then a column
-// operator (k_slice_rf.cu, whose sizes are compiled in):
-//     [D1 IFFT_R K1 FFT_R D1] (each row)  x  [D2 IFFT_r K2 FFT_r D2] (each column),
-// one launch each, a CTA per block of rows and per block of 16 columns.
+// The separable kinetic phase K1 K2 makes the transform part a row operator then
+// a column operator (k_slice_rf.cu, whose sizes are compiled in),
+//     Rot x [IFFT_r K2 FFT_r] (each column) x [IFFT_R K1 FFT_R] (each row) x Rot,
+// one launch each, a CTA per block of rows and per block of 16 columns; Rot(dt/2)
+// is applied as the row launch loads and as the column launch stores.
 //
 // The transforms are the Stockham transforms of k_slice.cu and k_lines.cu --
 // the same radices in the same order with the same complex64 twiddles -- with
 // the stages taken in two groups, each in registers.  A grid's rounding of its
 // twiddles shifts the wavepacket's norm by up to 1e-7 a step, either way and
-// different for each factorisation; keeping theirs keeps the results to the
-// random part of the rounding.  With n = A B, B the product of the first group:
+// different for each factorisation; keeping theirs (and Rot as the one rounded
+// product of its factors) keeps the results to the random part of the rounding.  With n = A B, B the product of the first group:
 //   pass 1, item a < A:  elements a + A b, the first group's B-point DFT -> slot a of block c
 //   pass 2, item c < B:  slots a of block c, the second group's A-point DFT with its
 //                        twiddles -> element c + B d
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan
   const bool en = p.esum != nullptr;
   double e_k = 0.0, e_r = 0.0;
 
-  with_group<BIG>(x.first, [&](auto gr) {                  // global, D -> X
+  with_group<BIG>(x.first, [&](auto gr) {             // global (ROWS: Rot) -> X
     typedef decltype(gr) G;
     constexpr int NB = G::r * G::rr;
     for (int e = tid; e < lines * A; e += NT) {
@@ -242,15 +243,18 @@ __global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan
       float2 v[NB];
 #pragma unroll
       for (int b = 0; b < NB; b++) v[b] = s[(long)(A * b) * gs];
+      if (KIND == ROWS) {
+        const float2 r2 = __ldg(p.rc2 + l * n2 + j0 + line);
 #pragma unroll
-      for (int b = 0; b < NB; b++) v[b] = cmul(v[b], d[a + A * b]);
+        for (int b = 0; b < NB; b++) v[b] = cmul(v[b], cmul(d[a + A * b], r2));
+      }
       First<G::r, G::rr, -1>::run(v);
 #pragma unroll
       for (int c = 0; c < NB; c++) X[line * xl + c * xb + a * xs] = v[c];
     }
   });
   __syncthreads();
-  with_group<BIG>(x.second, [&](auto gr) {                 // X -> K -> Y
+  with_group<BIG>(x.second, [&](auto gr) {            // X -> K -> Y
     typedef decltype(gr) G;
     constexpr int NA = G::r * G::rr;
     for (int e = tid; e < lines * B; e += NT) {
@@ -277,7 +281,7 @@ __global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan
     }
   });
   __syncthreads();
-  with_group<BIG>(x.first, [&](auto gr) {                  // Y -> X, inverse
+  with_group<BIG>(x.first, [&](auto gr) {             // Y -> X, inverse
     typedef decltype(gr) G;
     constexpr int NB = G::r * G::rr;
     for (int e = tid; e < lines * A; e += NT) {
@@ -293,7 +297,7 @@ __global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan
     }
   });
   __syncthreads();
-  with_group<BIG>(x.second, [&](auto gr) {                 // X, D -> global
+  with_group<BIG>(x.second, [&](auto gr) {            // X (COLS: Rot) -> global
     typedef decltype(gr) G;
     constexpr int NA = G::r * G::rr;
     for (int e = tid; e < lines * B; e += NT) {
@@ -305,9 +309,10 @@ __global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan
       for (int a = 0; a < NA; a++) v[a] = s[a * xs];
       second<G::r, G::rr, +1>(v, t + c, B);
       float2 *o = gb + (long)line * gl + (long)c * gs;
+      const float2 r1 = KIND == COLS ? __ldg(p.rc1 + l * n1 + q0 + line) : make_float2(1.f, 0.f);
 #pragma unroll
       for (int f = 0; f < NA; f++) {
-        v[f] = cmul(v[f], d[c + B * f]);
+        if (KIND == COLS) v[f] = cmul(v[f], cmul(r1, d[c + B * f]));
         o[(long)(B * f) * gs] = v[f];
       }
       if (KIND == COLS && en) {
