@@ -366,11 +366,8 @@ bool plan(int n1, int n2, Plan &out)
   Plan x{};
   if (!factor(n1, x.A1, x.B1) || !factor(n2, x.A2, x.B2)) return false;
   row_layout(x.A1, x.B1, sizeof(double2), x.bs, x.RS);
-  x.tc = 8;                                  // whole 128-byte segments
-  x.ncb = (n1 + x.tc - 1) / x.tc;
   x.mA1 = magic(x.A1);
   x.mB1 = magic(x.B1);
-  x.mQ = magic(x.tc);
   plans[{n1, n2}] = x;
   out = x;
   return true;
@@ -390,6 +387,12 @@ cudaError_t launch_axis_f64(const LineParams &p, cudaStream_t s)
   if (!plan(p.n1, p.n2, ax)) return cudaErrorInvalidValue;
   ax.hr = axis_rows(p.n1, p.n2, p.nruns * p.nl);
   ax.nrb = (p.n2 + ax.hr - 1) / ax.hr;
+  // columns of a tile: 16 where four CTAs' tiles still fit an SM and there are two CTAs
+  // per SM of them (step of 128 x 128 x 64 53.3 -> 51.3 us, of 4 runs of 144 x 120 x 64
+  // 196 -> 189), else 8, one 128-byte segment (72 x 192: 119 us, 123 with 16)
+  ax.tc = p.n2 <= 160 && (long)p.nruns * p.nl * ((p.n1 + 15) / 16) >= 296 ? 16 : 8;
+  ax.ncb = (p.n1 + ax.tc - 1) / ax.tc;
+  ax.mQ = magic(ax.tc);
   const cudaError_t e = launch_kind<ROWS>(p, ax, s);
   return e != cudaSuccess ? e : launch_kind<COLS>(p, ax, s);
 }

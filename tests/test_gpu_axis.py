@@ -59,3 +59,9 @@ def test_blocks_of_several_bases(prec, tol, monkeypatch):
     base = S.build_case("f+h2", 36, 30, 12, m=11, total_steps=6, n_energies=5, n_gradient_points=5)
     runs = [S.cs_case(base, J, K, 0, K + 1) for J, K in ((0, 0), (2, 1), (3, 3))]
     check(runs, 6, 3, monkeypatch, prec, tol)
+
+
+def test_fp64_wide_column_tiles(monkeypatch):
+    # enough slices for 16-column tiles, the last of them ragged (n1 = 72)
+    d = S.build_case("h+h2", 72, 30, 64, m=59, total_steps=3, n_energies=5, n_gradient_points=3)
+    check([d], 3, 3, monkeypatch, QD_PREC_FP64, 1e-10)
