@@ -20,7 +20,7 @@
 // k_mlp_adam sums the rows in order and updates the weights.  (One launch per
 // layer and direction, activations in global memory and the weight gradients
 // on 8 CTAs with atomics, took 342 us a step at 4096 samples; this form takes 22.)
-// Inference: one fused kernel per tile of 256 points (features from the
+// Inference: one fused kernel per tile of 512 points (features from the
 // Jacobi geometry, all layers in shared memory).
 #include <cmath>
 #include <cstring>
@@ -401,15 +401,16 @@ struct GridArgs {
 };
 // Every layer's weights stay in shared memory for the whole launch (loaded once
 // per CTA), activations of GP points at a time in place, transposed ([k][point]).
-// A thread forms 8 points x 4 outputs as paired FP32 FMAs (fma.rn.f32x2, two
-// points a register pair): per k, 2 16-byte loads of activations and 2 of
-// weights, which are stored twice each so that a pair (w, w) is one load, for 16
-// paired FMAs.  Bound: the products and the SiLUs together (12.4 kFMA per point,
-// 0.36 ms at the FP32 rate on 128 x 128 x 64, and 256 exponentials and divisions
-// a point, as many instructions as the paired FMAs).  There: scalar FMAs, 4 x 4
-// outputs a thread with scalar loads 1.18 ms; 8 x 4 with 16-byte loads 0.96 ms;
-// this form 0.91 ms.
-constexpr int GP = 256, GT = 512;
+// A thread forms 8 points x GP/64 outputs as paired FP32 FMAs (fma.rn.f32x2, two
+// points a register pair): at 512 points, per k, 2 16-byte loads of activations
+// and 2 of weights for 32 paired FMAs.  A 16-byte shared load costs four cycles of
+// the return path even when its lanes read one address, so loads per FMA are what
+// a tile is chosen by.  Bound: the products (12.4 kFMA per point, 0.36 ms at the FP32 rate on
+// 128 x 128 x 64) and the SiLUs (256 exponentials and divisions a point) together.
+// There: scalar FMAs, 4 x 4 outputs a thread with scalar loads 1.18 ms; 8 x 4 with
+// 16-byte loads 0.96; 8 x 4 paired, weights stored twice (a pair (w, w) one load)
+// 0.91, stored once 0.83; 8 x 8 0.77.
+constexpr int GT = 512;
 typedef unsigned long long f32x2;
 __device__ __forceinline__ f32x2 pack2(float a, float b)
 {
@@ -429,24 +430,26 @@ __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
+template <int GP>
 struct GridSmem {
-  float2 w[NL - 1][W][W];                 // layers 2..4: [k][o], each weight twice
+  float w[NL - 1][W][W];                  // layers 2..4: [k][o]
   float h[W][GP];                         // activations
   float w1[W][NF], b[NL][W], wo[W];
   float f[GP][NF];
   unsigned char mask[GP];
 };
+template <int GP>
 __global__ void __launch_bounds__(GT, 1) k_mlp_grid(GridArgs g, Norm nm, const float *wq,
                                                     double *pot, long npts, const double *r12p,
                                                     const double *r23p, const double *r13p)
 {
   extern __shared__ float4 grid_sm4[];
-  GridSmem &m = *reinterpret_cast<GridSmem *>(grid_sm4);
-  const int tid = threadIdx.x, tp = tid & 31, to = tid >> 5;   // points 4 tp.., 128 + 4 tp..; outputs 4 to..
+  GridSmem<GP> &m = *reinterpret_cast<GridSmem<GP> *>(grid_sm4);
+  constexpr int PO = GP / 64;             // outputs a thread
+  const int tid = threadIdx.x, tp = tid % (GP / 8), to = tid / (GP / 8);   // points 4 tp.., GP/2 + 4 tp..; outputs PO to..
   for (int x = tid; x < (NL - 1) * W * W; x += GT) {
     const int l = x / (W * W), k = x / W % W, o = x % W;
-    const float v = wq[layer_off(l + 1) + o * W + k];
-    m.w[l][k][o] = make_float2(v, v);
+    m.w[l][k][o] = wq[layer_off(l + 1) + o * W + k];
   }
   for (int x = tid; x < W * NF; x += GT) m.w1[x / NF][x % NF] = wq[x];
   for (int x = tid; x < NL * W; x += GT)
@@ -488,32 +491,37 @@ __global__ void __launch_bounds__(GT, 1) k_mlp_grid(GridArgs g, Norm nm, const f
     __syncthreads();
 #pragma unroll 1
     for (int l = 1; l < NL; l++) {
-      f32x2 acc[4][4];                    // point pairs x outputs
+      f32x2 acc[4][PO];                    // point pairs x outputs
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float bj = m.b[l][4 * to + j];
+      for (int j = 0; j < PO; j++) {
+        const float bj = m.b[l][PO * to + j];
 #pragma unroll
         for (int i = 0; i < 4; i++) acc[i][j] = pack2(bj, bj);
       }
-#pragma unroll 4
+#pragma unroll 2
       for (int k = 0; k < W; k++) {
         const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(&m.h[k][4 * tp]);
         const ulonglong2 a1 = *reinterpret_cast<const ulonglong2 *>(&m.h[k][GP / 2 + 4 * tp]);
-        const ulonglong2 w0 = *reinterpret_cast<const ulonglong2 *>(&m.w[l - 1][k][4 * to]);
-        const ulonglong2 w1 = *reinterpret_cast<const ulonglong2 *>(&m.w[l - 1][k][4 * to + 2]);
-        const f32x2 a[4] = {a0.x, a0.y, a1.x, a1.y}, w[4] = {w0.x, w0.y, w1.x, w1.y};
+        const f32x2 a[4] = {a0.x, a0.y, a1.x, a1.y};
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+        for (int j = 0; j < PO; j += 4) {
+          const float4 w4 = *reinterpret_cast<const float4 *>(&m.w[l - 1][k][PO * to + j]);
+          const float w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] = fma2(a[i], w[j], acc[i][j]);
+          for (int c = 0; c < 4; c++) {
+            const f32x2 ww = pack2(w[c], w[c]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[i][j + c] = fma2(a[i], ww, acc[i][j + c]);
+          }
+        }
       }
       __syncthreads();                    // every read of the activations is done
 #pragma unroll
-      for (int j = 0; j < 4; j++)
+      for (int j = 0; j < PO; j++)
 #pragma unroll
         for (int i = 0; i < 4; i += 2) {
           const float2 u = unpack2(acc[i][j]), v = unpack2(acc[i + 1][j]);
-          *reinterpret_cast<float4 *>(&m.h[4 * to + j][(i ? GP / 2 : 0) + 4 * tp]) =
+          *reinterpret_cast<float4 *>(&m.h[PO * to + j][(i ? GP / 2 : 0) + 4 * tp]) =
               make_float4(silu(u.x), silu(u.y), silu(v.x), silu(v.y));
         }
       __syncthreads();
@@ -541,15 +549,29 @@ __global__ void __launch_bounds__(GT, 1) k_mlp_grid(GridArgs g, Norm nm, const f
   }
 }
 
+template <int GP>
+cudaError_t run_mlp_grid(const GridArgs &g, const Norm &nm, const float *wq, double *pot, long npts,
+                         const double *r12p, const double *r23p, const double *r13p)
+{
+  const cudaError_t e = cudaFuncSetAttribute(
+      k_mlp_grid<GP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GridSmem<GP>));
+  if (e != cudaSuccess) return e;
+  const long blocks = (npts + GP - 1) / GP;
+  k_mlp_grid<GP><<<(unsigned)(blocks < 148 ? blocks : 148), GT, sizeof(GridSmem<GP>)>>>(
+      g, nm, wq, pot, npts, r12p, r23p, r13p);
+  return cudaSuccess;
+}
 cudaError_t launch_mlp_grid(const GridArgs &g, const Norm &nm, const float *wq, double *pot,
                             long npts, const double *r12p, const double *r23p, const double *r13p)
 {
-  const cudaError_t e = cudaFuncSetAttribute(
-      k_mlp_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GridSmem));
+  // A round of 512-point tiles over the 148 SMs takes 1.85 times one of 256-point
+  // tiles (55 and 30 us), which are taken where fewer SMs idle with them: 5000 points
+  // 48 us against 81, 163 840 157 against 171, but 1 048 576 827 against 767.
+  const long r512 = (npts + 148 * 512 - 1) / (148 * 512), r256 = (npts + 148 * 256 - 1) / (148 * 256);
+  const cudaError_t e = 13 * r512 <= 7 * r256
+                            ? run_mlp_grid<512>(g, nm, wq, pot, npts, r12p, r23p, r13p)
+                            : run_mlp_grid<256>(g, nm, wq, pot, npts, r12p, r23p, r13p);
   if (e != cudaSuccess) return e;
-  const long blocks = (npts + GP - 1) / GP;
-  k_mlp_grid<<<(unsigned)(blocks < 148 ? blocks : 148), GT, sizeof(GridSmem)>>>(
-      g, nm, wq, pot, npts, r12p, r23p, r13p);
   qd_count_launches(1);
   return cudaGetLastError();
 }

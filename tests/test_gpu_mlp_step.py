@@ -57,3 +57,16 @@ def test_adam_steps(n, batch):
             s0, total, seen = 0, 0.0, 0
     assert np.linalg.norm(w - p) < 1e-3
     assert abs(loss - last) < 1e-3 * last
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 148 * 256, 148 * 256 + 1, 148 * 512 + 1, 200001])
+def test_energies_at_the_edges_of_a_round(n):
+    # an FP32 output sums 64 products with relative rounding near 1e-7 over four layers
+    data = training_set(S.leps_f_h2(), MASSES, n=n, seed=23)
+    with Surrogate(seed=7) as sur:
+        w, _ = sur.params()
+        norm = np.array([0.2, 0.3, 0.05, 0.2, 0.3, 0.1, 0.05, 0.1], dtype=np.float32)
+        sur.set_params(w, norm)
+        got = sur(*data[:3])
+    ref = M.predict(w, norm, *data[:3])
+    assert np.abs(got - ref).max() < 1e-5 * np.abs(ref).max() + 1e-7
