@@ -15,11 +15,11 @@
 //
 // A training step is two launches.  k_mlp_step takes tiles of 32 samples
 // through the whole network in shared memory, forward and backward, with all
-// weights beside them; the weight gradients of a CTA's tiles stay in registers
-// (49 per thread) and go out once, as that CTA's row of a partial array.
+// weights beside them; the weight gradients of a CTA's tiles are summed in that
+// CTA's row of a partial array.
 // k_mlp_adam sums the rows in order and updates the weights.  (One launch per
 // layer and direction, activations in global memory and the weight gradients
-// on 8 CTAs with atomics, took 342 us a step at 4096 samples; this form takes 22.)
+// on 8 CTAs with atomics, took 342 us a step at 4096 samples; this form takes 20.)
 // Inference: one fused kernel per tile of 512 points (features from the
 // Jacobi geometry, all layers in shared memory).
 #include <cmath>
@@ -72,13 +72,15 @@ __global__ void k_features(int n, const double *r12, const double *r23, const do
 // Forward and backward over samples [0, n) in tiles of TS, one CTA to a tile at
 // a time: part[blockIdx][0..NPARAM) = this CTA's share of d(mean squared
 // error)/d(parameters) (GRADS), part[blockIdx][NPARAM] its sum of squared errors.
-// 256 threads; a layer's 32 x 64 outputs are 2 samples x 4 outputs a thread with
-// the contraction read four at a time (6 16-byte loads per 32 FMAs), its weight
-// gradient 4 x 4 entries a thread over the 32 samples (2 per 16).
-// Bound: the latency of the chain of layers at two warps per scheduler (one
-// tile of a 4096-sample batch per CTA: 9200 FMAs per scheduler, 4 us at the FMA
-// rate, in about 16 us); smaller tiles would not fill more SMs by much and
-// double the weight traffic per sample.
+// 256 threads; a layer's 32 x 64 outputs are 4 samples x 4 outputs a thread over
+// one half of the contraction, read four at a time (4 16-byte loads per 32 FMAs;
+// 2 x 4 outputs over all of it, 6 loads, took 22.0 us a step at 4096 samples,
+// halves 20.6), its weight gradient 4 x 4 entries a thread over the 32 samples
+// (2 per 16), straight to the partial row, so that the backward layers are one loop
+// (unrolled, with 48 sums in registers, the step waited for instructions: 19.8).
+// Bound: the return path of the shared-memory loads (19 000 cycles of one tile's
+// 16-byte loads at four cycles each, 10 us; the FMAs take 4 us); smaller tiles
+// would not fill more SMs by much and double the weight traffic per sample.
 constexpr int TS = 32;                    // samples of a tile
 constexpr int LDA = W + 4;                // row stride: 16-byte rows, conflict-free quarter-warps
 constexpr int PSTRIDE = (NPARAM + 1 + 3) / 4 * 4;
@@ -86,10 +88,28 @@ struct StepSmem {
   float w[NL - 1][W][LDA];                // layers 2..4
   float a[NL][TS][LDA], s[NL][TS][LDA];   // activations, SiLU'(z)
   float d[2][TS][LDA];                    // backward signal, ping-pong
+  float x[8][256];                        // halves of a contraction, exchanged
   float f[TS][4];                         // features, and 1 for the bias
   float e[TS];                            // 2 (y - t) / n_total
   float w1[W][NF], b[NL][W], wo[W];
 };
+
+// Adds the two halves of a contraction: thread tid holds 4 x 4 partial sums, and of
+// their total rows 2 kh, 2 kh + 1 go to z (the other two rows to thread tid ^ 128).
+// Between two calls stands the block barrier at the end of a layer.
+__device__ __forceinline__ void exchange(StepSmem &m, int kh, int tid, const float (&acc)[4][4],
+                                         float (&z)[2][4])
+{
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) m.x[4 * i + j][tid ^ 128] = kh ? acc[i][j] : acc[2 + i][j];
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 2; i++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) z[i][j] = (kh ? acc[2 + i][j] : acc[i][j]) + m.x[4 * i + j][tid];
+}
 
 template <bool GRADS>
 __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, const float *F,
@@ -100,9 +120,15 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
   StepSmem &m = *reinterpret_cast<StepSmem *>(step_sm4);
   __shared__ float red[8];
   const int tid = threadIdx.x, tr = tid >> 4, tc = tid & 15;
+  const int kh = tid >> 7, tq = tr & 7;   // half of a contraction, its first sample
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");     // the weights: the last step's update
+  float fr[NF];                           // features of a tile's sample tid, read ahead
+#define QD_FEATURES(s0)                                                    \
+  _Pragma("unroll") for (int c = 0; c < NF; c++)                           \
+    fr[c] = tid < TS && (s0) + tid < n ? F[(long)((s0) + tid) * NF + c] : 0.f
   {                                       // 16-byte weight rows, all loads in flight together
+    static_assert(NL * W == 256 && W * NF <= 256, "one bias and one first weight a thread");
     constexpr int PT = W * W / 4 / 256;
     float4 v[NL - 1][PT];
 #pragma unroll
@@ -110,6 +136,9 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
 #pragma unroll
       for (int q = 0; q < PT; q++)
         v[l - 1][q] = reinterpret_cast<const float4 *>(w + layer_off(l))[tid + 256 * q];
+    const float v1 = tid < W * NF ? w[tid] : 0.f, vo = tid < W ? w[OFF_WO + tid] : 0.f;
+    const float vb = w[layer_off(tid / W) + W * (tid / W ? W : NF) + tid % W];
+    QD_FEATURES((int)blockIdx.x * TS);
 #pragma unroll
     for (int l = 1; l < NL; l++)
 #pragma unroll
@@ -117,27 +146,21 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
         const int x = tid + 256 * q;
         *reinterpret_cast<float4 *>(&m.w[l - 1][x / (W / 4)][4 * (x % (W / 4))]) = v[l - 1][q];
       }
+    if (tid < W * NF) m.w1[tid / NF][tid % NF] = v1;
+    m.b[tid / W][tid % W] = vb;
+    if (tid < W) m.wo[tid] = vo;
   }
-  for (int x = tid; x < W * NF; x += 256) m.w1[x / NF][x % NF] = w[x];
-  for (int x = tid; x < NL * W; x += 256)
-    m.b[x / W][x % W] = w[layer_off(x / W) + W * (x / W ? W : NF) + x % W];
-  if (tid < W) m.wo[tid] = w[OFF_WO + tid];
   const float bo = w[OFF_BO];
   static_assert(layer_off(1) % 4 == 0 && (W * W + W) % 4 == 0, "16-byte weight rows");
 
-  float g[NL - 1][4][4] = {};             // dW of layers 2..4, entries [4 tr + i][4 tc + j]
+  float *out = part + (size_t)blockIdx.x * PSTRIDE;
   float g1 = 0.f;                         // layer 1: dW[tid / 4][tid % 4], the bias at 3
-  float gb[NL - 1] = {};                  // biases of layers 2..4 (tid < 64)
   float go = 0.f, gbo = 0.f;              // output weight tid - 64 and its bias
   float l2 = 0.f;
   for (int s0 = blockIdx.x * TS; s0 < n; s0 += gridDim.x * TS) {
-    if (tid < TS) {
-      const bool ok = s0 + tid < n;
-      const float *f = F + (long)(s0 + tid) * NF;
-#pragma unroll
-      for (int c = 0; c < NF; c++) m.f[tid][c] = ok ? f[c] : 0.f;
-      m.f[tid][3] = 1.f;
-    }
+    if (tid < TS) *reinterpret_cast<float4 *>(m.f[tid]) = make_float4(fr[0], fr[1], fr[2], 1.f);
+    const float tgt = s0 + (tid >> 3) < n ? target[s0 + (tid >> 3)] : 0.f;   // of the output stage
+    QD_FEATURES(s0 + (int)gridDim.x * TS);
     __syncthreads();                      // features (and, first time, the weights) in place
     {                                     // layer 1: output o of samples s
       const int o = tid & (W - 1);
@@ -152,31 +175,35 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
     __syncthreads();
 #pragma unroll 1
     for (int l = 1; l < NL; l++) {
-      float acc[2][4];
+      float acc[4][4];
 #pragma unroll
-      for (int i = 0; i < 2; i++)
+      for (int i = 0; i < 4; i++)
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = m.b[l][tc + 16 * j];
+        for (int j = 0; j < 4; j++) acc[i][j] = kh ? 0.f : m.b[l][tc + 16 * j];
 #pragma unroll
-      for (int k = 0; k < W; k += 4) {
-        float4 a[2], v[4];
+      for (int k4 = 0; k4 < W / 2; k4 += 4) {
+        const int k = kh * (W / 2) + k4;
+        float4 a[4], v[4];
 #pragma unroll
-        for (int i = 0; i < 2; i++) a[i] = *reinterpret_cast<const float4 *>(&m.a[l - 1][tr + 16 * i][k]);
+        for (int i = 0; i < 4; i++) a[i] = *reinterpret_cast<const float4 *>(&m.a[l - 1][tq + 8 * i][k]);
 #pragma unroll
         for (int j = 0; j < 4; j++) v[j] = *reinterpret_cast<const float4 *>(&m.w[l - 1][tc + 16 * j][k]);
 #pragma unroll
-        for (int i = 0; i < 2; i++)
+        for (int i = 0; i < 4; i++)
 #pragma unroll
           for (int j = 0; j < 4; j++)
             acc[i][j] = fmaf(a[i].w, v[j].w, fmaf(a[i].z, v[j].z,
                         fmaf(a[i].y, v[j].y, fmaf(a[i].x, v[j].x, acc[i][j]))));
       }
+      float z[2][4];
+      exchange(m, kh, tid, acc, z);
 #pragma unroll
       for (int i = 0; i < 2; i++)
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-          m.a[l][tr + 16 * i][tc + 16 * j] = silu(acc[i][j]);
-          if (GRADS) m.s[l][tr + 16 * i][tc + 16 * j] = dsilu(acc[i][j]);
+          const int s = tq + 8 * (2 * kh + i);
+          m.a[l][s][tc + 16 * j] = silu(z[i][j]);
+          if (GRADS) m.s[l][s][tc + 16 * j] = dsilu(z[i][j]);
         }
       __syncthreads();
     }
@@ -189,7 +216,7 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
         for (int i = 0; i < 4; i++) acc = fmaf(m.a[NL - 1][s][k + i], m.wo[k + i], acc);
 #pragma unroll
       for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-      const float d = s0 + s < n ? acc + bo - target[s0 + s] : 0.f;
+      const float d = s0 + s < n ? acc + bo - tgt : 0.f;
       const float e = 2.f * d * inv_total;
       if ((tid & 7) == 0) {
         l2 = fmaf(d, d, l2);
@@ -209,10 +236,21 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
         go = fmaf(m.e[s], m.a[NL - 1][s][tid - W], go);
         gbo += m.e[s];
       }
-#pragma unroll
+    const bool more = s0 != (int)blockIdx.x * TS;     // a tile after the CTA's first
+#pragma unroll 1
     for (int l = NL - 1; l >= 1; l--) {
       float (*D)[LDA] = m.d[(NL - 1 - l) & 1], (*Dp)[LDA] = m.d[(NL - l) & 1];
-      // dW[o][k] = sum_s D[s][o] A[s][k]
+      // dW[o][k] += sum_s D[s][o] A[s][k], entries [4 tr + i][4 tc + j]; the bias: tid < 64
+      float *gw = out + layer_off(l) + 4 * tr * W + 4 * tc, *gbp = out + layer_off(l) + W * W + tid;
+      float g[4][4] = {}, gb = 0.f;
+      if (more) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+          const float4 t = *reinterpret_cast<const float4 *>(gw + i * W);
+          g[i][0] = t.x; g[i][1] = t.y; g[i][2] = t.z; g[i][3] = t.w;
+        }
+        if (tid < W) gb = *gbp;
+      }
 #pragma unroll 16
       for (int s = 0; s < TS; s++) {
         const float4 x = *reinterpret_cast<const float4 *>(&D[s][4 * tr]);
@@ -221,22 +259,28 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) g[l - 1][i][j] = fmaf(xs[i], ys[j], g[l - 1][i][j]);
+          for (int j = 0; j < 4; j++) g[i][j] = fmaf(xs[i], ys[j], g[i][j]);
       }
-      if (tid < W)
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+        *reinterpret_cast<float4 *>(gw + i * W) = make_float4(g[i][0], g[i][1], g[i][2], g[i][3]);
+      if (tid < W) {
 #pragma unroll 8
-        for (int s = 0; s < TS; s++) gb[l - 1] += D[s][tid];
-      // D below: (sum_o D[s][o] W[o][k]) SiLU'(z[s][k]), samples tr, tr + 16, k = 4 tc + j
-      float acc[2][4] = {};
+        for (int s = 0; s < TS; s++) gb += D[s][tid];
+        *gbp = gb;
+      }
+      // D below: (sum_o D[s][o] W[o][k]) SiLU'(z[s][k]), k = 4 tc + j
+      float acc[4][4] = {}, y[2][4];
 #pragma unroll
-      for (int o = 0; o < W; o += 4) {
-        float4 x[2], v[4];
+      for (int o4 = 0; o4 < W / 2; o4 += 4) {
+        const int o = kh * (W / 2) + o4;
+        float4 x[4], v[4];
 #pragma unroll
-        for (int i = 0; i < 2; i++) x[i] = *reinterpret_cast<const float4 *>(&D[tr + 16 * i][o]);
+        for (int i = 0; i < 4; i++) x[i] = *reinterpret_cast<const float4 *>(&D[tq + 8 * i][o]);
 #pragma unroll
         for (int q = 0; q < 4; q++) v[q] = *reinterpret_cast<const float4 *>(&m.w[l - 1][o + q][4 * tc]);
 #pragma unroll
-        for (int i = 0; i < 2; i++) {
+        for (int i = 0; i < 4; i++) {
           const float xs[4] = {x[i].x, x[i].y, x[i].z, x[i].w};
 #pragma unroll
           for (int q = 0; q < 4; q++) {
@@ -247,12 +291,13 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
           }
         }
       }
+      exchange(m, kh, tid, acc, y);
 #pragma unroll
       for (int i = 0; i < 2; i++) {
-        const int s = tr + 16 * i;
+        const int s = tq + 8 * (2 * kh + i);
         const float4 z = *reinterpret_cast<const float4 *>(&m.s[l - 1][s][4 * tc]);
         *reinterpret_cast<float4 *>(&Dp[s][4 * tc]) =
-            make_float4(acc[i][0] * z.x, acc[i][1] * z.y, acc[i][2] * z.z, acc[i][3] * z.w);
+            make_float4(y[i][0] * z.x, y[i][1] * z.y, y[i][2] * z.z, y[i][3] * z.w);
       }
       __syncthreads();
     }
@@ -261,7 +306,8 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
     __syncthreads();                      // before the next tile's features
   }
 
-  float *out = part + (size_t)blockIdx.x * PSTRIDE;
+#undef QD_FEATURES
+
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) l2 += __shfl_xor_sync(0xffffffffu, l2, o);
   if ((tid & 31) == 0) red[tid >> 5] = l2;
@@ -272,14 +318,6 @@ __global__ void __launch_bounds__(256, 1) k_mlp_step(int n, float inv_total, con
     out[NPARAM] = t;
   }
   if (!GRADS) return;
-#pragma unroll
-  for (int l = 1; l < NL; l++) {
-#pragma unroll
-    for (int i = 0; i < 4; i++)
-      *reinterpret_cast<float4 *>(out + layer_off(l) + (4 * tr + i) * W + 4 * tc) =
-          make_float4(g[l - 1][i][0], g[l - 1][i][1], g[l - 1][i][2], g[l - 1][i][3]);
-    if (tid < W) out[layer_off(l) + W * W + tid] = gb[l - 1];
-  }
   if ((tid & 3) < NF) out[(tid >> 2) * NF + (tid & 3)] = g1;
   else out[W * NF + (tid >> 2)] = g1;
   if (tid >= W && tid < 2 * W) out[OFF_WO + tid - W] = go;
