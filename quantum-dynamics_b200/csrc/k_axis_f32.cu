@@ -1,6 +1,6 @@
 // k_axis_f32.cu -- the l-space part of one complex64 split-operator step for any
 // grid whose sizes are two groups of one or two radices (every even product of
-// 2, 3 and 5 up to 250 but 162, and 256):
+// 2, 3 and 5 from 6 to 256 but 8 and 162, some larger and some odd ones):
 //     psi_l <- Rot(dt/2) IFFT2 [exp(-i(T1+T2)dt)/(n1 n2)] FFT2 Rot(dt/2) psi_l
 // (evolution_dt, timeEvol.C:625-635; tables timeEvol.C:465-517).
 //
@@ -15,7 +15,8 @@
 // the stages taken in two groups, each in registers.  A grid's rounding of its
 // twiddles shifts the wavepacket's norm by up to 1e-7 a step, either way and
 // different for each factorisation; keeping theirs (and Rot as the one rounded
-// product of its factors) keeps the results to the random part of the rounding.  With n = A B, B the product of the first group:
+// product of its factors) keeps the results to the random part of the rounding.
+// With n = A B, B the product of the first group:
 //   pass 1, item a < A:  elements a + A b, the first group's B-point DFT -> slot a of block c
 //   pass 2, item c < B:  slots a of block c, the second group's A-point DFT with its
 //                        twiddles -> element c + B d
@@ -25,9 +26,9 @@
 // element, was what the other kernels spent their time on.
 //
 // Bound: the latency of four dependent passes per CTA and two launches for grids
-// of a few hundred slices, then L2 (8 runs of 96 x 96 x 48: 113 MB in 54 us).
+// of a few hundred slices, then L2 (8 runs of 96 x 96 x 48: 113 MB in 45 us).
 // Per step, best Stockham form -> this: 3 runs of 108 x 90 x 50 99 -> 26 us,
-// 144 x 120 x 64 52 -> 25 us, 200 x 180 x 40 93 -> 29 us.
+// 144 x 120 x 64 52 -> 24 us, 200 x 180 x 40 93 -> 30 us.
 #include <algorithm>
 #include <map>
 #include <mutex>

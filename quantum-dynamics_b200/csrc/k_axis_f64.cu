@@ -21,8 +21,8 @@
 //
 // Bound: HBM, or L2 for states that stay there (256 x 192 x 128: 403 MB in 122 us,
 // half the measured copy rate).  Per step, Stockham kernels -> these (events
-// around the launches): 256 x 192 x 128 471 -> 122 us, 128 x 128 x 64 98 -> 28 us,
-// 64 x 64 x 39 38 -> 15 us, 100 x 54 x 29 50 -> 18 us.
+// around the launches): 256 x 192 x 128 471 -> 122 us, 128 x 128 x 64 98 -> 25 us,
+// 64 x 64 x 39 38 -> 15 us, 100 x 54 x 29 50 -> 15 us.
 #include <algorithm>
 #include <map>
 #include <mutex>

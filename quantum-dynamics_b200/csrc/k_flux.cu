@@ -8,7 +8,7 @@
 //                  recurrence of timeEvol.C:807-817 evaluated directly, FP64)
 //   k_flux_gemm    phi_E += sum_t dt e^{iE t} psi_s(t), dphi_E likewise
 //                  (PsiTimeToPsiEnergyOnSurface, CRPAux.F:4-31): a
-//                  register-tiled complex FP64 GEMM over the chunk.
+//                  complex GEMM over the chunk on the FP64 tensor cores.
 //   k_crp          P(E) = Im(sum_k w_k sum_i conj(phi) dphi) / eta^2 dr1/mu2
 //                  (CalculateCRP, CRPAux.F:34-66), warp-shuffle reduction.
 #include "qd_kernels.h"

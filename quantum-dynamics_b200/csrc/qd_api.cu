@@ -955,9 +955,9 @@ bool axis_f64(const qd_handle *h)
 //     CTAs per slice, timed on the handle's zero l-space buffer (a zero
 //     wavepacket stays zero), the choice kept for later handles of the shapes;
 //   sizes that k_axis_f32.cu / k_axis_f64.cu take: those (complex64, us a step,
-//     the best Stockham form -> k_axis_f32: 48 x 40 x 24 16.3 -> 16.5, 54 x 60 x 32
-//     25 -> 17.5, 144 x 120 x 64 52 -> 25, 200 x 180 x 40 93 -> 36, 8 runs of
-//     96 x 96 x 48 105 -> 54; FP64: k_axis_f64.cu);
+//     the best Stockham form -> k_axis_f32: 48 x 40 x 24 16.3 -> 14.7, 54 x 60 x 32
+//     25 -> 16, 144 x 120 x 64 52 -> 24, 200 x 180 x 40 93 -> 30, 8 runs of
+//     96 x 96 x 48 105 -> 45; FP64: k_axis_f64.cu);
 //   other grids: FP64 the split kernels; complex64 the split kernels or the
 //     Stockham slice kernel on 1, 2 or 4 CTAs per slice, timed likewise.
 // QD_SLICE_CLUSTER=0|1|2|4|8|9|10|11|12 forces a choice (0 the split kernels,
