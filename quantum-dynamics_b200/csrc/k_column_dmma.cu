@@ -1,6 +1,6 @@
 // k_column_dmma.cu -- the FP64 column pass on the FP64 tensor cores.
 //
-// Per tile of 16 grid columns, the work of k_column.cu (B, absorber, surface
+// Per tile of 8 grid columns, the work of k_column.cu (B, absorber, surface
 // rows, norm, exp(-iVdt), F) as two GEMMs of mma.sync m16n8k8 .f64.  One
 // 16-row operand holds eight grid columns: rows 0-7 their real parts, rows
 // 8-15 their imaginary parts, so the thread that gets an accumulator's real
@@ -17,12 +17,15 @@
 // m16n8k8, one warp per scheduler or more; plain DFMA chains 34).  FP64
 // operands need 8 x 8 values in registers per thread to keep plain FMAs fed
 // from shared memory; with mma the warps of an SM read about 64 B a clock.
-// Tile of 16 columns, not 32: two tiles fit beside P at 128 x 128, one per group
-// of warps, and grids of a few hundred tiles spread over the SMs.  Per launch,
-// against the SIMT kernel: 256 x 192 x 128 (6.4 GFLOP) 835 -> 235 us, 128 x 128 x
-// 64 87 -> 35 us, 64 x 64 x 40 30 -> 14 us (each with 5 us of event and launch time).
+// Four groups of four warps an SM with a tile of 8 columns each, so that every
+// scheduler has a warp of each and one group's loads, phases and stores run under
+// the others' products; two groups of eight warps with 16 columns left the tensor
+// pipe idle longer (256 x 192 x 128: 235 us against 228, step of 128 x 128 x 64 51.1
+// against 48.1).  Per launch, against the SIMT kernel: 256 x 192 x 128 (6.4 GFLOP)
+// 835 -> 228 us, 128 x 128 x 64 87 -> 33 us, 64 x 64 x 40 30 -> 14 us (each with 5 us
+// of event and launch time).
 //
-// Shared layouts: a tile is [row][17] complex (17: every 16-byte access of a
+// Shared layouts: a tile is [row][9] complex (9: every 16-byte access of a
 // warp touches the eight bank groups evenly); P is [k][nlp], nlp a multiple of
 // 16, with the 16-byte units of row k permuted by XOR (swz) so that both the
 // pair loads along l (GEMM1) and the loads down k (GEMM2) are free of conflicts.
@@ -30,8 +33,10 @@
 
 namespace {
 
-constexpr int TC = 16;          // grid columns of a tile
+constexpr int TC = 8;           // grid columns of a tile
 constexpr int LD = TC + 1;      // tile row stride (complex)
+constexpr int WN = 4;           // warps of a group: its tile's outputs are theirs in turn
+constexpr int GT = 32 * WN;     // threads of a group
 constexpr int MAXGRP = 16;      // groups of eight angles or orders
 
 __device__ __forceinline__ void dmma(double (&c)[4], const double2 a0, const double2 a1,
@@ -63,20 +68,18 @@ inline size_t dmma_smem(int nth, int nl, int tiles)
          sizeof(double) * pad8(nth);
 }
 
-// acc[m][n] = tile (columns 8 m + g) x P over kb blocks of 8 contraction
+// acc[n] = tile (column g) x P over kb blocks of 8 contraction
 // indices; the warp's n-th output group: rows 8 (wn + WN n) + ... of the result.
 // The XOR of P's units changes with a block's parity only (GEMM1) or not at
 // all (GEMM2), so a lane's addresses advance by constants.
-template <int MI, int NI, int WN, bool FWD>
-__device__ __forceinline__ void gemm(double (&acc)[MI][NI][4], const double2 *tile, const double *P,
+template <int NI, bool FWD>
+__device__ __forceinline__ void gemm(double (&acc)[NI][4], const double2 *tile, const double *P,
                                      int nlp, int kb, int ngrp, int wn, int g, int t)
 {
 #pragma unroll
-  for (int m = 0; m < MI; m++)
+  for (int n = 0; n < NI; n++)
 #pragma unroll
-    for (int n = 0; n < NI; n++)
-#pragma unroll
-      for (int i = 0; i < 4; i++) acc[m][n][i] = 0.0;
+    for (int i = 0; i < 4; i++) acc[n][i] = 0.0;
   const double2 *row = tile + 2 * t * LD + g;
   const double *pk[NI];                 // FWD: P[2t][8 grp + g]; else P[8 grp + g][..]
   int o0[NI], o1[NI];                   // FWD: rows 2t, 2t + 1; else even, odd block
@@ -95,12 +98,7 @@ __device__ __forceinline__ void gemm(double (&acc)[MI][NI][4], const double2 *ti
     }
   }
   auto block = [&](int b) {
-    double2 a[MI][2];
-#pragma unroll
-    for (int m = 0; m < MI; m++) {
-      a[m][0] = row[8 * m];
-      a[m][1] = row[LD + 8 * m];
-    }
+    const double2 a0 = row[0], a1 = row[LD];
     row += 8 * LD;
 #pragma unroll
     for (int n = 0; n < NI; n++) {
@@ -116,8 +114,7 @@ __device__ __forceinline__ void gemm(double (&acc)[MI][NI][4], const double2 *ti
         b1 = v.y;
         if (b & 1) pk[n] += 16;
       }
-#pragma unroll
-      for (int m = 0; m < MI; m++) dmma(acc[m][n], a[m][0], a[m][1], b0, b1);
+      dmma(acc[n], a0, a1, b0, b1);
     }
   };
   int b = 0;
@@ -130,13 +127,11 @@ __device__ __forceinline__ void gemm(double (&acc)[MI][NI][4], const double2 *ti
   for (; b < kb; b++) block(b);
 }
 
-// NG groups of 2 x 4 warps, each with its own tiles and its own barrier: one
-// group's loads, theta-space work and stores overlap the other's products.  In
-// a group warp (wm, wn) takes 8 of the tile's columns and every fourth group of
-// eight outputs, NI of them.
-constexpr int WN = 4, GT = 256;         // warps along the outputs, threads of a group
+// NG groups of four warps, each with its own tiles and its own barrier: one
+// group's loads, theta-space work and stores overlap the others' products.  In
+// a group warp wn takes every fourth group of eight outputs, NI of them.
 template <int NG, int NI, int MODE>
-__global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
+__global__ void __launch_bounds__(NG * GT, 4 / NG) k_column_dmma(ColumnParams p)
 {
   constexpr int NT = NG * GT;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -147,7 +142,7 @@ __global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
   double2 *cur = reinterpret_cast<double2 *>(smem) + grp * rows * LD;   // the group's tile [rows][LD]
   double *P = reinterpret_cast<double *>(reinterpret_cast<double2 *>(smem) + NG * rows * LD);
   double *w = P + nthp * nlp;
-  const int wn = (gtid >> 5) % WN, c0 = 8 * ((gtid >> 5) / WN);   // the warp's first column
+  const int wn = gtid >> 5;
   const int n12 = (int)p.n12;
   const int tpr = (n12 + TC - 1) / TC;                // tiles per run
   const int ntiles = tpr * p.nruns;
@@ -155,8 +150,7 @@ __global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
   pdl_trigger();
 
   auto group_sync = [&] {
-    if (NG == 1) __syncthreads();
-    else asm volatile("bar.sync %0, %1;" :: "r"(1 + grp), "r"(GT) : "memory");
+    asm volatile("bar.sync %0, %1;" :: "r"(1 + grp), "r"(GT) : "memory");
   };
   auto run_at = [&](int at) { return p.run_order ? p.run_order[at] : at; };
   auto load_P = [&](int set) {                        // by the whole CTA
@@ -214,10 +208,10 @@ __global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
       asm volatile("cp.async.wait_group 0;" ::: "memory");
       group_sync();                                   // the tile in place
 
-      double acc[1][NI][4];
+      double acc[NI][4];
       if (MODE != COL_HEAD) {
         // exp(-iVdt) of this thread's values, in flight during GEMM1
-        const int q = p0 + c0 + g;
+        const int q = p0 + g;
         const bool in = q < n12;
         double2 ph[NI][2];
         if (MODE == COL_MID) {
@@ -228,7 +222,7 @@ __global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
             for (int i = 0; i < 2; i++)
               if (k0 + 8 * WN * n + i < p.nth && in) ph[n][i] = __ldg(v + (long)(8 * WN * n + i) * n12);
         }
-        gemm<1, NI, WN, false>(acc, cur + c0, P, nlp, lgrp, kgrp, wn, g, t);
+        gemm<NI, false>(acc, cur, P, nlp, lgrp, kgrp, wn, g, t);
         group_sync();                                 // every read of the l-space tile is done
         if (MODE == COL_TAIL) fetch(mine);
         const int j = in ? q / p.n1 : 0, i1 = in ? q - j * p.n1 : 0;
@@ -242,7 +236,7 @@ __global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
 #pragma unroll
           for (int i = 0; i < 2; i++) {
             const int k = k0 + 8 * WN * n + i;
-            double2 v = make_double2(acc[0][n][i], acc[0][n][2 + i]);
+            double2 v = make_double2(acc[n][i], acc[n][2 + i]);
             if (k < p.nth && in) {
               const double wk = w[k];
               if (p.esum)
@@ -255,7 +249,7 @@ __global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
             } else {
               v = make_double2(0.0, 0.0);
             }
-            if (MODE == COL_MID) cur[k * LD + c0 + g] = v;
+            if (MODE == COL_MID) cur[k * LD + g] = v;
           }
         }
         if (MODE == COL_TAIL) continue;
@@ -282,10 +276,10 @@ __global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
         }
       }
       group_sync();                                   // the theta-space tile in place
-      gemm<1, NI, WN, true>(acc, cur + c0, P, nlp, kgrp, lgrp, wn, g, t);
+      gemm<NI, true>(acc, cur, P, nlp, kgrp, lgrp, wn, g, t);
       group_sync();                                   // every read of it is done
       fetch(mine);
-      const int q = p0 + c0 + g;
+      const int q = p0 + g;
       if (q < n12) {
         double2 *dst = reinterpret_cast<double2 *>(p.lpsi) + ((long)run * p.nl + k0) * p.n12 + q;
 #pragma unroll
@@ -295,7 +289,7 @@ __global__ void __launch_bounds__(NG * GT, 2 / NG) k_column_dmma(ColumnParams p)
             const int l = k0 + 8 * WN * n + i;
             if (l < p.nl)
               dst[(long)(8 * WN * n + i) * n12] =
-                  make_double2((l + 0.5) * acc[0][n][i], (l + 0.5) * acc[0][n][2 + i]);
+                  make_double2((l + 0.5) * acc[n][i], (l + 0.5) * acc[n][2 + i]);
           }
       }
     }
@@ -318,10 +312,10 @@ cudaError_t launch(const ColumnParams &p, cudaStream_t s)
   cudaError_t e = cudaFuncSetAttribute(k_column_dmma<NG, NI, MODE>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
   if (e != cudaSuccess) return e;
-  const long ntiles = (p.n12 + TC - 1) / TC * p.nruns;
-  const long slots = NG == 1 && sm <= 113 * 1024 ? 2 * 148 : 148;    // CTAs resident at once
+  const long ctas = ((p.n12 + TC - 1) / TC * p.nruns + NG - 1) / NG;  // a tile for every group
+  const long slots = 148 * (4 / NG);                  // CTAs resident at once
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(ntiles < slots ? ntiles : slots));
+  cfg.gridDim = dim3((unsigned)(ctas < slots ? ctas : slots));
   cfg.blockDim = dim3(NG * GT);
   cfg.dynamicSmemBytes = sm;
   cfg.stream = s;
@@ -345,18 +339,17 @@ template <int NG, int NI> cudaError_t launch_mode(const ColumnParams &p, int mod
 
 }  // namespace
 
-// P and two tiles in shared memory, and no more than MAXGRP groups on either side
+// P and four tiles in shared memory, and no more than MAXGRP groups on either side
 bool column_dmma_ok(int nth, int nl)
 {
-  return pad8(nth) <= 8 * MAXGRP && pad8(nl) <= 8 * MAXGRP && dmma_smem(nth, nl, 2) <= 227 * 1024;
+  return pad8(nth) <= 8 * MAXGRP && pad8(nl) <= 8 * MAXGRP && dmma_smem(nth, nl, 4) <= 227 * 1024;
 }
 
 cudaError_t launch_column_dmma(const ColumnParams &p, int mode, cudaStream_t s)
 {
-  // 64 angles and orders or fewer: P and a tile take 50 KB at most, two CTAs of one
-  // group share an SM (128 x 128 x 64: 35.1 us a launch; one CTA of two groups 33.2,
-  // but 64 x 64 x 40 14.4 against 13.9); more: one CTA of two groups (256 x 192 x 128:
-  // 235 us; one group of 16 warps with the next tile in a second buffer 256)
-  return pad8(p.nth) <= 64 && pad8(p.nl) <= 64 ? launch_mode<1, 2>(p, mode, s)
-                                               : launch_mode<2, 4>(p, mode, s);
+  // 64 angles and orders or fewer: P and two tiles take 51 KB at most, and two CTAs
+  // of two groups share an SM (step of 128 x 128 x 64 48.1 us; one CTA of four groups
+  // 49.6, four of one group 57.7, as four copies of P are loaded); more: one CTA
+  return pad8(p.nth) <= 64 && pad8(p.nl) <= 64 ? launch_mode<2, 2>(p, mode, s)
+                                               : launch_mode<4, 4>(p, mode, s);
 }
