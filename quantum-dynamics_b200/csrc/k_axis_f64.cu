@@ -61,6 +61,8 @@ template <int MAXR, typename F> __device__ __forceinline__ void with_radix(int r
 // kernels by the larger radix of their dimension, as its values take the
 // registers (step of 200 x 180 x 40 82 -> 76 us, of 3 runs of 108 x 90 x 50 79 -> 76,
 // against one kernel for both dimensions and all radices up to 16)
+// 11 to 16: four CTAs, 128 registers (256 x 192 x 128 123 us; five at 102 registers 124,
+// three at 168 137; 128 x 128 x 64 25, 28 and 32)
 template <int KIND, int MAXR>
 __global__ void __launch_bounds__(NT, MAXR > 16 ? 2 : MAXR > 10 ? 4 : 5) k_axis_f64(LineParams p, Plan ax)
 {

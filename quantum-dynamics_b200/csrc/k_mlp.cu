@@ -20,8 +20,9 @@
 // k_mlp_adam sums the rows in order and updates the weights.  (One launch per
 // layer and direction, activations in global memory and the weight gradients
 // on 8 CTAs with atomics, took 342 us a step at 4096 samples; this form takes 20.)
-// Inference: one fused kernel per tile of 512 points (features from the
+// Inference: one fused kernel per tile of 64 to 512 points (features from the
 // Jacobi geometry, all layers in shared memory).
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -439,7 +440,7 @@ struct GridArgs {
 };
 // Every layer's weights stay in shared memory for the whole launch (loaded once
 // per CTA), activations of GP points at a time in place, transposed ([k][point]).
-// A thread forms 8 points x GP/64 outputs as paired FP32 FMAs (fma.rn.f32x2, two
+// A thread forms 8 points (4 in tiles below 256) x 2, 4 or 8 outputs as paired FP32 FMAs (fma.rn.f32x2, two
 // points a register pair): at 512 points, per k, 2 16-byte loads of activations
 // and 2 of weights for 32 paired FMAs.  A 16-byte shared load costs four cycles of
 // the return path even when its lanes read one address, so loads per FMA are what
@@ -483,8 +484,10 @@ __global__ void __launch_bounds__(GT, 1) k_mlp_grid(GridArgs g, Norm nm, const f
 {
   extern __shared__ float4 grid_sm4[];
   GridSmem<GP> &m = *reinterpret_cast<GridSmem<GP> *>(grid_sm4);
-  constexpr int PO = GP / 64;             // outputs a thread
-  const int tid = threadIdx.x, tp = tid % (GP / 8), to = tid / (GP / 8);   // points 4 tp.., GP/2 + 4 tp..; outputs PO to..
+  constexpr int PP = GP < 256 ? 4 : 8, PO = GP * W / (GT * PP);   // points and outputs a thread
+  constexpr int WV = PO < 4 ? PO : 4;     // weights of a load
+  // points 4 tp.. (and GP/2 + 4 tp..), outputs PO to..
+  const int tid = threadIdx.x, tp = tid % (GP / PP), to = tid / (GP / PP);
   for (int x = tid; x < (NL - 1) * W * W; x += GT) {
     const int l = x / (W * W), k = x / W % W, o = x % W;
     m.w[l][k][o] = wq[layer_off(l + 1) + o * W + k];
@@ -529,27 +532,37 @@ __global__ void __launch_bounds__(GT, 1) k_mlp_grid(GridArgs g, Norm nm, const f
     __syncthreads();
 #pragma unroll 1
     for (int l = 1; l < NL; l++) {
-      f32x2 acc[4][PO];                    // point pairs x outputs
+      f32x2 acc[PP / 2][PO];               // point pairs x outputs
 #pragma unroll
       for (int j = 0; j < PO; j++) {
         const float bj = m.b[l][PO * to + j];
 #pragma unroll
-        for (int i = 0; i < 4; i++) acc[i][j] = pack2(bj, bj);
+        for (int i = 0; i < PP / 2; i++) acc[i][j] = pack2(bj, bj);
       }
 #pragma unroll 2
       for (int k = 0; k < W; k++) {
-        const ulonglong2 a0 = *reinterpret_cast<const ulonglong2 *>(&m.h[k][4 * tp]);
-        const ulonglong2 a1 = *reinterpret_cast<const ulonglong2 *>(&m.h[k][GP / 2 + 4 * tp]);
-        const f32x2 a[4] = {a0.x, a0.y, a1.x, a1.y};
+        f32x2 a[PP / 2];
 #pragma unroll
-        for (int j = 0; j < PO; j += 4) {
-          const float4 w4 = *reinterpret_cast<const float4 *>(&m.w[l - 1][k][PO * to + j]);
-          const float w[4] = {w4.x, w4.y, w4.z, w4.w};
+        for (int i = 0; i < PP / 2; i += 2) {
+          const ulonglong2 v = *reinterpret_cast<const ulonglong2 *>(&m.h[k][(i ? GP / 2 : 0) + 4 * tp]);
+          a[i] = v.x;
+          a[i + 1] = v.y;
+        }
 #pragma unroll
-          for (int c = 0; c < 4; c++) {
+        for (int j = 0; j < PO; j += WV) {
+          float w[WV];
+          if constexpr (WV == 4) {
+            const float4 v = *reinterpret_cast<const float4 *>(&m.w[l - 1][k][PO * to + j]);
+            w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+          } else {
+            const float2 v = *reinterpret_cast<const float2 *>(&m.w[l - 1][k][PO * to + j]);
+            w[0] = v.x; w[1] = v.y;
+          }
+#pragma unroll
+          for (int c = 0; c < WV; c++) {
             const f32x2 ww = pack2(w[c], w[c]);
 #pragma unroll
-            for (int i = 0; i < 4; i++) acc[i][j + c] = fma2(a[i], ww, acc[i][j + c]);
+            for (int i = 0; i < PP / 2; i++) acc[i][j + c] = fma2(a[i], ww, acc[i][j + c]);
           }
         }
       }
@@ -557,7 +570,7 @@ __global__ void __launch_bounds__(GT, 1) k_mlp_grid(GridArgs g, Norm nm, const f
 #pragma unroll
       for (int j = 0; j < PO; j++)
 #pragma unroll
-        for (int i = 0; i < 4; i += 2) {
+        for (int i = 0; i < PP / 2; i += 2) {
           const float2 u = unpack2(acc[i][j]), v = unpack2(acc[i + 1][j]);
           *reinterpret_cast<float4 *>(&m.h[PO * to + j][(i ? GP / 2 : 0) + 4 * tp]) =
               make_float4(silu(u.x), silu(u.y), silu(v.x), silu(v.y));
@@ -602,13 +615,15 @@ cudaError_t run_mlp_grid(const GridArgs &g, const Norm &nm, const float *wq, dou
 cudaError_t launch_mlp_grid(const GridArgs &g, const Norm &nm, const float *wq, double *pot,
                             long npts, const double *r12p, const double *r23p, const double *r13p)
 {
-  // A round of 512-point tiles over the 148 SMs takes 1.85 times one of 256-point
-  // tiles (55 and 30 us), which are taken where fewer SMs idle with them: 5000 points
-  // 48 us against 81, 163 840 157 against 171, but 1 048 576 827 against 767.
-  const long r512 = (npts + 148 * 512 - 1) / (148 * 512), r256 = (npts + 148 * 256 - 1) / (148 * 256);
-  const cudaError_t e = 13 * r512 <= 7 * r256
-                            ? run_mlp_grid<512>(g, nm, wq, pot, npts, r12p, r23p, r13p)
-                            : run_mlp_grid<256>(g, nm, wq, pot, npts, r12p, r23p, r13p);
+  // The tile whose rounds over the 148 SMs take least: a launch takes 10 us and 12,
+  // 16.5, 28 or 52 us a round of 64, 128, 256 or 512 points an SM (512 points 22, 26, 38
+  // and 62 us, 303 104 386, 268, 235 and 219).  Costs in half microseconds.
+  auto cost = [&](long points, long half_us) { return (npts + 148 * points - 1) / (148 * points) * half_us; };
+  const long t64 = cost(64, 24), t128 = cost(128, 33), t256 = cost(256, 56), t512 = cost(512, 104);
+  const long least = std::min(std::min(t64, t128), std::min(t256, t512));
+  const auto run = least == t512 ? run_mlp_grid<512> : least == t256 ? run_mlp_grid<256>
+                 : least == t128 ? run_mlp_grid<128> : run_mlp_grid<64>;
+  const cudaError_t e = run(g, nm, wq, pot, npts, r12p, r23p, r13p);
   if (e != cudaSuccess) return e;
   qd_count_launches(1);
   return cudaGetLastError();

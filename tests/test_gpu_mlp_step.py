@@ -59,7 +59,7 @@ def test_adam_steps(n, batch):
     assert abs(loss - last) < 1e-3 * last
 
 
-@pytest.mark.parametrize("n", [1, 255, 257, 148 * 256, 148 * 256 + 1, 148 * 512 + 1, 200001])
+@pytest.mark.parametrize("n", [1, 63, 255, 257, 148 * 64, 148 * 64 + 1, 148 * 128 + 1, 148 * 256, 148 * 256 + 1, 148 * 512 + 1, 200001])
 def test_energies_at_the_edges_of_a_round(n):
     # an FP32 output sums 64 products with relative rounding near 1e-7 over four layers
     data = training_set(S.leps_f_h2(), MASSES, n=n, seed=23)
