@@ -130,7 +130,9 @@ inline bool all_finite(const double *a, size_t n)
 // copy engine moves each chunk as soon as it is staged, so the host copy of
 // chunk c overlaps the transfer of chunk c - 1.  One transfer at a time per
 // process; without page-locked memory the copies fall back to plain
-// cudaMemcpyAsync from the caller's arrays.
+// cudaMemcpyAsync from the caller's arrays.  The buffers serve every device; the
+// events that guard them belong to one each, as an event can only be recorded on
+// a stream of its own device.
 class Staging {
  public:
   static constexpr size_t CHUNK = size_t(32) << 20;   // bytes per staging buffer
@@ -184,7 +186,7 @@ class Staging {
     size_t done = 0;                             // doubles of array i already staged
     while (i < np) {
       const int b = (int)(next_++ % NBUF);
-      cudaError_t e = cudaEventSynchronize(ev_[b]);   // the buffer's last transfer is done
+      cudaError_t e = wait(b);   // the buffer's last transfer is done
       if (e != cudaSuccess) return e;
       size_t co = 0;                             // bytes of the buffer in use
       while (i < np) {
@@ -208,7 +210,7 @@ class Staging {
         co = (co + m * w + 63) & ~size_t(63);    // each part starts 64-byte aligned
         if (co >= CHUNK) break;
       }
-      e = cudaEventRecord(ev_[b], st);
+      e = mark(b, st);
       if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -258,14 +260,14 @@ class Staging {
     };
     auto issue = [&](size_t c) -> cudaError_t {
       const int b = (int)(c % NBUF);
-      cudaError_t e = cudaEventSynchronize(ev_[b]);
+      cudaError_t e = wait(b);
       each_part(c, [&](int i, size_t po, size_t co, size_t n) {
         if (e == cudaSuccess)
           e = cudaMemcpyAsync(static_cast<char *>(buf_[b]) + co,
                               static_cast<const char *>(pc[i].src) + po, n,
                               cudaMemcpyDeviceToHost, st);
       });
-      if (e == cudaSuccess) e = cudaEventRecord(ev_[b], st);
+      if (e == cudaSuccess) e = mark(b, st);
       return e;
     };
     for (size_t c = 0; c < nch && c < (size_t)NBUF - 1; c++) {
@@ -274,7 +276,7 @@ class Staging {
     }
     for (size_t c = 0; c < nch; c++) {
       const int b = (int)(c % NBUF);
-      cudaError_t e = cudaEventSynchronize(ev_[b]);
+      cudaError_t e = wait(b);
       if (e != cudaSuccess) return e;
       each_part(c, [&](int i, size_t po, size_t co, size_t n) {
         if (pc[i].widen)
@@ -296,18 +298,40 @@ class Staging {
 
  private:
   Staging() = default;
+  // the buffers, and the current device's events, exist (made on first use)
   bool ready()
   {
-    if (tried_) return ok_;
-    tried_ = true;
-    ok_ = true;
-    for (int b = 0; b < NBUF && ok_; b++)
-      ok_ = cudaHostAlloc(&buf_[b], CHUNK, cudaHostAllocPortable) == cudaSuccess &&
-            cudaEventCreateWithFlags(&ev_[b], cudaEventDisableTiming) == cudaSuccess;
-    if (ok_)
-      for (int b = 0; b < NBUF && ok_; b++) ok_ = cudaEventRecord(ev_[b], 0) == cudaSuccess;
-    if (!ok_) cudaGetLastError();
-    return ok_;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= MAXDEV) {
+      cudaGetLastError();
+      return false;
+    }
+    if (!tried_) {
+      tried_ = ok_ = true;
+      for (int b = 0; b < NBUF && ok_; b++)
+        ok_ = cudaHostAlloc(&buf_[b], CHUNK, cudaHostAllocPortable) == cudaSuccess;
+    }
+    if (ok_ && !dev_tried_[dev]) {
+      dev_tried_[dev] = dev_ok_[dev] = true;
+      for (int b = 0; b < NBUF && dev_ok_[dev]; b++)
+        dev_ok_[dev] = cudaEventCreateWithFlags(&ev_[dev][b], cudaEventDisableTiming) == cudaSuccess;
+    }
+    if (!ok_ || !dev_ok_[dev]) {
+      cudaGetLastError();
+      return false;
+    }
+    return true;
+  }
+  // buffer b's last transfer, whichever device it was on, is done
+  cudaError_t wait(int b) { return last_[b] ? cudaEventSynchronize(last_[b]) : cudaSuccess; }
+  // buffer b's last transfer is the one issued on st, a stream of the current device
+  cudaError_t mark(int b, cudaStream_t st)
+  {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    last_[b] = ev_[dev][b];
+    return cudaEventRecord(last_[b], st);
   }
   // memcpy over the host pool, the stores streamed past the caches where the
   // destination is 16-byte aligned (no read of the destination lines); with
@@ -413,8 +437,9 @@ class Staging {
     });
   }
   std::mutex mu_;
-  bool tried_ = false, ok_ = false;
+  static constexpr int MAXDEV = 64;
+  bool tried_ = false, ok_ = false, dev_tried_[MAXDEV] = {}, dev_ok_[MAXDEV] = {};
   void *buf_[NBUF] = {};
-  cudaEvent_t ev_[NBUF] = {};
+  cudaEvent_t ev_[MAXDEV][NBUF] = {}, last_[NBUF] = {};
   size_t next_ = 0;               // the upload's next staging buffer (round robin)
 };
