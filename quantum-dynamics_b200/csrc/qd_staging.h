@@ -240,7 +240,8 @@ class Staging {
       widen = widen || pc[i].widen;
     }
     if (widen && !ready()) return cudaErrorMemoryAllocation;
-    if (!widen && (!ready() || (np == 1 && total < least))) {
+    // (the size first: a small array alone needs no staging buffers, and makes none)
+    if (!widen && ((np == 1 && total < least) || !ready())) {
       for (int i = 0; i < np; i++) {
         cudaError_t e = cudaMemcpyAsync(pc[i].dst, pc[i].src, pc[i].bytes, cudaMemcpyDeviceToHost,
                                         st);

@@ -51,3 +51,21 @@ def test_devices_in_turn(tmp_path, first, second):
       }
       return 0;
     }""" % (first, second, first))
+
+
+def test_small_fetch_pins_nothing(tmp_path):
+    run(tmp_path, """
+    int main() {
+      Staging &s = Staging::get();
+      const V a = ramp(1000);
+      V b(a.size());
+      CHECK(s.download(b.data(), a.data(), 8 * a.size(), nullptr) == cudaSuccess);
+      CHECK(b == a);
+      CHECK(fake::pinned == 0);
+      const V big = ramp(Staging::LARGE / 8);       // the smallest array that is staged
+      V c(big.size());
+      CHECK(s.download(c.data(), big.data(), 8 * big.size(), nullptr) == cudaSuccess);
+      CHECK(c == big);
+      CHECK(fake::pinned == (long)(Staging::NBUF * Staging::CHUNK));
+      return 0;
+    }""")
