@@ -127,12 +127,9 @@ int qd_set_error(int code, const char *msg)
 }
 void qd_count_launches(int n) { g_launches += n; }
 
-// staged from 2 MB on: below, the copy threads cost more than they take off the faults
-// of a fresh result array (a surface call with 1.2 MB 405 us staged, 260 not, with 1.3 MB 470 and 300)
 cudaError_t qd_fetch(void *dst, const void *src, size_t bytes)
 {
-  const Staging::Piece one{dst, src, bytes};
-  return Staging::get().download(&one, 1, 0, size_t(2) << 20);
+  return Staging::get().fetch(dst, src, bytes);
 }
 
 // call scratch (qd_err.h): one pool per device, made on first use

@@ -35,8 +35,8 @@ inline int qd_errf(int code, const char *fmt, ...)
 constexpr size_t QD_SCRATCH_KEEP = size_t(256) << 20;
 cudaError_t qd_scratch_alloc(void **p, size_t bytes);
 // device -> host on the legacy default stream, through the page-locked staging
-// buffers and the host threads from 256 KiB on (a fresh result array's page
-// faults are then shared by the threads too); returns when dst holds the data
+// buffers and the host threads from 2 MB on (a fresh result array's page faults
+// are then shared by the threads too); returns when dst holds the data
 cudaError_t qd_fetch(void *dst, const void *src, size_t bytes);
 struct qd_scratch {
   void *p = nullptr;

@@ -69,3 +69,40 @@ def test_small_fetch_pins_nothing(tmp_path):
       CHECK(fake::pinned == (long)(Staging::NBUF * Staging::CHUNK));
       return 0;
     }""")
+
+
+@pytest.mark.parametrize("mib", [1, 3, 8])
+def test_waiting_for_a_kernel_delays_no_other_copy(tmp_path, mib):
+    # a fetch whose kernel is still running (the stream's synchronise does not return)
+    # leaves the staging buffers to another thread's copies
+    run(tmp_path, """
+    #include <chrono>
+    int main() {
+      Staging &s = Staging::get();
+      const V a = ramp((size_t(%d) << 20) / 8), up = ramp((size_t(8) << 20) / 8);
+      std::mutex m;
+      std::condition_variable cv;
+      bool waiting = false, uploaded = false, in_time = false;
+      fake::on_stream_sync = [&] {
+        std::unique_lock<std::mutex> l(m);
+        if (waiting) return;                       // the fetch's first wait: its kernel
+        waiting = true;
+        cv.notify_all();
+        in_time = cv.wait_for(l, std::chrono::seconds(10), [&] { return uploaded; });
+      };
+      V got(a.size()), dst(up.size());
+      cudaError_t e = cudaErrorInvalidValue;
+      std::thread t([&] { e = s.fetch(got.data(), a.data(), 8 * a.size()); });
+      {
+        std::unique_lock<std::mutex> l(m);
+        CHECK(cv.wait_for(l, std::chrono::seconds(10), [&] { return waiting; }));
+      }
+      const Staging::Up u{dst.data(), up.data(), up.size(), false, true};
+      std::vector<char> bad;
+      CHECK(s.upload(&u, 1, nullptr, bad) == cudaSuccess);
+      { std::lock_guard<std::mutex> l(m); uploaded = true; }
+      cv.notify_all();
+      t.join();
+      CHECK(in_time && e == cudaSuccess && got == a && dst == up);
+      return 0;
+    }""" % mib)
