@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstring>
 #include <cuda_runtime.h>
+#include <exception>
 #include <functional>
 #include <mutex>
 #include <thread>
@@ -18,7 +19,7 @@
 
 // Host worker threads for the input checks and the staging copies: created
 // once per process (up to 16, the calling thread included) and reused, so a
-// 32 MiB chunk costs no thread creation.  run(fn) calls fn(t) for every
+// 32 MiB chunk costs no thread creation; fewer where the system refuses more.  run(fn) calls fn(t) for every
 // worker t and returns when all are done; callers take turns.  In a process
 // forked after the pool was made (its workers do not exist there) the calling
 // thread does every part itself.
@@ -56,7 +57,12 @@ class HostPool {
   {
     const unsigned hw = std::thread::hardware_concurrency();
     const unsigned n = std::max(1u, std::min(16u, hw ? hw : 1u));
-    for (unsigned t = 1; t < n; t++) th_.emplace_back([this, t] { loop(t); });
+    try {
+      th_.reserve(n);
+      for (unsigned t = 1; t < n; t++) th_.emplace_back([this, t] { loop(t); });
+    } catch (const std::exception &) {
+      // the system refuses more threads: the ones there are and the caller do the work
+    }
   }
   void loop(unsigned t)
   {

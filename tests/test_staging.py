@@ -106,3 +106,25 @@ def test_waiting_for_a_kernel_delays_no_other_copy(tmp_path, mib):
       CHECK(in_time && e == cudaSuccess && got == a && dst == up);
       return 0;
     }""" % mib)
+
+
+@pytest.mark.parametrize("threads", [0, 1, 5])
+def test_fewer_worker_threads_than_asked_for(tmp_path, threads):
+    # the system gives `threads` threads and refuses the others
+    run(tmp_path, """
+    #include <cerrno>
+    #include <dlfcn.h>
+    #include <pthread.h>
+    static int given = 0;
+    extern "C" int pthread_create(pthread_t *t, const pthread_attr_t *a, void *(*f)(void *), void *p) {
+      typedef int (*Fn)(pthread_t *, const pthread_attr_t *, void *(*)(void *), void *);
+      static Fn real = (Fn)dlsym(RTLD_NEXT, "pthread_create");
+      return given < %d ? (given++, real(t, a, f, p)) : EAGAIN;
+    }
+    int main() {
+      const V a = ramp((size_t(5) << 20) / 8);
+      V b(a.size());
+      CHECK(Staging::get().fetch(b.data(), a.data(), 8 * a.size()) == cudaSuccess);
+      CHECK(b == a && given <= %d && all_finite(a.data(), a.size()));
+      return 0;
+    }""" % (threads, threads), "-rdynamic", "-D_GNU_SOURCE")
