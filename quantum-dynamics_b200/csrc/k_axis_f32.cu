@@ -40,6 +40,7 @@ namespace {
 
 enum Kind { ROWS = 0, COLS = 1 };
 constexpr int NT = 128;               // threads per CTA
+constexpr int STATIC_SMEM = 32 * sizeof(double);   // of the energy sums
 constexpr int TCOLS = 16;             // columns of a tile: whole 128-byte segments
 
 // one dimension: stages (r1, r2) then (r3, r4); r2 = r4 = 1 for single-stage groups
@@ -179,7 +180,7 @@ template <int KIND, bool BIG>
 __global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan ax)
 {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double red[32];
+  __shared__ double red[STATIC_SMEM / sizeof(double)];
   const int tid = threadIdx.x;
   const int n1 = p.n1, n2 = p.n2;
   const int per_slice = KIND == ROWS ? ax.nrb : ax.ncb;
@@ -344,8 +345,7 @@ template <int KIND, bool BIG> cudaError_t launch_one(const LineParams &p, const 
 {
   const size_t sm = sizeof(float2) * (KIND == ROWS ? (size_t)ax.hr * (ax.RS + ax.RY) + 3 * p.n1
                                                    : 2 * (size_t)p.n2 * TCOLS + 3 * p.n2);
-  cudaError_t e = cudaFuncSetAttribute(k_axis_f32<KIND, BIG>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const cudaError_t e = allow_smem(k_axis_f32<KIND, BIG>, STATIC_SMEM);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   const int per = KIND == ROWS ? ax.nrb : ax.ncb;

@@ -33,6 +33,7 @@ namespace {
 
 enum Kind { ROWS = 0, COLS = 1 };
 constexpr int NT = 128;                               // threads per CTA
+constexpr int STATIC_SMEM = 32 * sizeof(double);      // of the energy sums
 
 // factors of a grid, row layout and block sizes
 struct Plan {
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(NT, MAXR > 16 ? 2 : MAXR > 10 ? 4 : 5) k_axis_
 {
   typedef double2 C;
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ double red[32];
+  __shared__ double red[STATIC_SMEM / sizeof(double)];
   const int tid = threadIdx.x;
   const int n1 = p.n1, n2 = p.n2, A1 = ax.A1, B1 = ax.B1, A2 = ax.A2, B2 = ax.B2;
   const int bs = ax.bs, RS = ax.RS;
@@ -276,8 +277,7 @@ template <int KIND, int MAXR>
 cudaError_t launch_one(const LineParams &p, const Plan &ax, cudaStream_t s)
 {
   const size_t sm = smem_bytes<KIND>(ax, p.n1, p.n2);
-  cudaError_t e = cudaFuncSetAttribute(k_axis_f64<KIND, MAXR>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const cudaError_t e = allow_smem(k_axis_f64<KIND, MAXR>, STATIC_SMEM);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   const int per = KIND == ROWS ? ax.nrb : ax.ncb;

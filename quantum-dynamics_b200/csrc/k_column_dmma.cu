@@ -309,8 +309,7 @@ template <int NG, int NI, int MODE>
 cudaError_t launch(const ColumnParams &p, cudaStream_t s)
 {
   const size_t sm = dmma_smem(p.nth, p.nl, NG);
-  cudaError_t e = cudaFuncSetAttribute(k_column_dmma<NG, NI, MODE>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+  const cudaError_t e = allow_smem(k_column_dmma<NG, NI, MODE>);
   if (e != cudaSuccess) return e;
   const long ctas = ((p.n12 + TC - 1) / TC * p.nruns + NG - 1) / NG;  // a tile for every group
   const long slots = 148 * (4 / NG);                  // CTAs resident at once

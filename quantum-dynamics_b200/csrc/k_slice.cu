@@ -197,9 +197,7 @@ __global__ void __launch_bounds__(NT, 1) k_slice(LineParams p)
 template <int CL> cudaError_t launch_cl(const LineParams &p, cudaStream_t s)
 {
   const size_t sm = slice_smem_bytes(p.n1, p.n2, CL);
-  const void *kern = reinterpret_cast<const void *>(&k_slice<CL>);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sm);
+  const cudaError_t e = allow_smem(k_slice<CL>);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.nruns * p.nl * CL + p.flux_ctas));
@@ -213,9 +211,7 @@ template <int CL> cudaError_t launch_cl(const LineParams &p, cudaStream_t s)
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  LineParams pc = p;
-  void *args[] = {&pc};
-  return cudaLaunchKernelExC(&cfg, kern, args);
+  return cudaLaunchKernelEx(&cfg, k_slice<CL>, p);
 }
 
 }  // namespace

@@ -222,6 +222,16 @@ struct CrpParams {
   double *crp;
 };
 
+// Lets a kernel whose shared memory depends on the grid be launched with all that a
+// block can have (227 KB less its static shared memory).  Never the grid's own size:
+// the limit belongs to the kernel and the device, and another thread may launch the
+// same kernel for another grid between this call and the launch.
+template <typename K> cudaError_t allow_smem(K *kernel, int static_bytes = 0)
+{
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              227 * 1024 - static_bytes);
+}
+
 // launchers (return cudaGetLastError() after the launch)
 template <typename R> cudaError_t launch_column(const ColumnParams &p, int mode, cudaStream_t s);
 // FP64 column pass on the tensor cores; the bases it takes

@@ -18,11 +18,11 @@
 #endif
 
 // Host worker threads for the input checks and the staging copies: created
-// once per process (up to 16, the calling thread included) and reused, so a
-// 32 MiB chunk costs no thread creation; fewer where the system refuses more.  run(fn) calls fn(t) for every
-// worker t and returns when all are done; callers take turns.  In a process
-// forked after the pool was made (its workers do not exist there) the calling
-// thread does every part itself.
+// once per process (up to 16, the calling thread included; fewer where the
+// system refuses more) and reused, so a 32 MiB chunk costs no thread creation.
+// run(fn) calls fn(t) for every worker t and returns when all are done; callers
+// take turns.  In a process forked after the pool was made (its workers do not
+// exist there) the calling thread does every part itself.
 class HostPool {
  public:
   static HostPool &get()
