@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan
   };
   const int lines = KIND == ROWS ? nr : TCOLS;
   // energy step: this thread's shares of sum T |FFT|^2 and (COLS) of sum (I1 + I2) |psi_l|^2,
-  // as in k_slice_rf.cu
+  // squared in FP64 like the split kernels' (k_lines.cu)
   const bool en = p.esum != nullptr;
   double e_k = 0.0, e_r = 0.0;
 
@@ -270,8 +270,10 @@ __global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan
       if (en) {
         const double *T = KIND == ROWS ? p.T1 : p.T2;
 #pragma unroll
-        for (int f = 0; f < NA; f++)
-          e_k += (double)(v[f].x * v[f].x + v[f].y * v[f].y) * __ldg(T + c + B * f);
+        for (int f = 0; f < NA; f++) {
+          const double2 z = to_z(v[f]);
+          e_k += (z.x * z.x + z.y * z.y) * __ldg(T + c + B * f);
+        }
       }
       // (the scale 1 / (n1 n2) on the values, not in the table: a rounded table entry
       // would scale its frequency alike on every step)
@@ -320,8 +322,10 @@ __global__ void __launch_bounds__(NT, BIG ? 5 : 8) k_axis_f32(LineParams p, Plan
       if (KIND == COLS && en) {
         const double i1 = __ldg(p.I1 + q0 + line);
 #pragma unroll
-        for (int f = 0; f < NA; f++)
-          e_r += (double)(v[f].x * v[f].x + v[f].y * v[f].y) * (i1 + __ldg(p.I2 + c + B * f));
+        for (int f = 0; f < NA; f++) {
+          const double2 z = to_z(v[f]);
+          e_r += (z.x * z.x + z.y * z.y) * (i1 + __ldg(p.I2 + c + B * f));
+        }
       }
     }
   });
