@@ -357,13 +357,15 @@ SLICE_KINDS = {0: "split row and column kernels", 1: "Stockham cluster kernel, 1
                9: "register-FFT kernel k_slice_rf, 2-CTA clusters",
                10: "register-FFT kernel k_slice_rf, 4-CTA clusters",
                11: "register-FFT kernel k_slice_rf, 4-CTA clusters, 16x16 row transforms",
-               12: "run-time register-FFT kernels k_axis_f32, rows then columns"}
+               12: "run-time register-FFT kernels {axis}, rows then columns"}
 
 
 def describe_choice(ch, fp64):
     """The autotuners' picks for the timed handle (qd_kernel_choice)."""
-    return {"l_space": "FP64 run-time register-FFT kernels k_axis_f64" if fp64 else SLICE_KINDS.get(ch[0], str(ch[0])),
-            "column": "tensor cores (k_column_tc, tcgen05 kind::f16)" if ch[1] else "SIMT",
+    axis, tc = ("k_axis_f64", "k_column_dmma, mma.sync f64") if fp64 else \
+        ("k_axis_f32", "k_column_tc, tcgen05 kind::f16")
+    return {"l_space": SLICE_KINDS.get(ch[0], str(ch[0])).format(axis=axis),
+            "column": f"tensor cores ({tc})" if ch[1] else "SIMT",
             "flux_gemm_variant": ch[2],
             "flux_full_chunks": "chirp-z (k_flux_czt)" if ch[3] else "direct GEMM (k_flux_gemm)"}
 

@@ -1611,8 +1611,8 @@ int qd_set_profiling(qd_handle *h, int32_t on)
 int qd_kernel_choice(qd_handle *h, int32_t out[4])
 {
   if (!h || !out) return set_err(QD_ERR_INVALID, "NULL argument");
-  out[0] = h->prec == QD_PREC_FP32 ? h->slice_cluster : 0;
-  out[1] = h->use_tc ? 1 : 0;
+  out[0] = h->slice_cluster;
+  out[1] = (h->prec == QD_PREC_FP32 ? h->use_tc : column_dmma_ok(h->nth, h->nl)) ? 1 : 0;
   out[2] = h->flux_variant;
   out[3] = h->d_czt_b ? 1 : 0;
   return QD_OK;
