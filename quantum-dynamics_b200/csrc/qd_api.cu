@@ -540,83 +540,6 @@ bool axis_f64(const qd_handle *h)
   return !(force && atoi(force) == 0) && axis_f64_ok(h->n1, h->n2);
 }
 
-// Choice of the l-space kernel.
-//   complex64, sizes compiled in: the register-FFT slice kernel on 1, 2 or 4
-//     CTAs per slice, timed on the handle's zero l-space buffer (a zero
-//     wavepacket stays zero), the choice kept for later handles of the shapes;
-//   sizes that k_axis_f32.cu / k_axis_f64.cu take: those (complex64, us a step,
-//     the best Stockham form -> k_axis_f32: 48 x 40 x 24 16.3 -> 14.7, 54 x 60 x 32
-//     25 -> 16, 144 x 120 x 64 52 -> 24, 200 x 180 x 40 93 -> 30, 8 runs of
-//     96 x 96 x 48 105 -> 45; FP64: k_axis_f64.cu);
-//   other grids: FP64 the split kernels; complex64 the split kernels or the
-//     Stockham slice kernel on 1, 2 or 4 CTAs per slice, timed likewise.
-// QD_SLICE_CLUSTER=0|1|2|4|8|9|10|11|12 forces a choice (0 the split kernels,
-// 1, 2, 4 the Stockham slice kernel, 8, 9, 10 the register-FFT kernel on 1, 2
-// and 4 CTAs, 11 its wide form, 12 the run-time register-FFT kernels; FP64 knows
-// 0 and 12 only).
-int tune_slice(qd_handle *h)
-{
-  const bool f32 = h->prec == QD_PREC_FP32;
-  h->slice_cluster = !f32 && axis_f64(h) ? SLICE_AX : 0;
-  if (!f32) return QD_OK;
-  auto built = [&](int cl) { return slice_cluster_ok(h->n1, h->n2, cl) != 0; };
-  if (const char *force = getenv("QD_SLICE_CLUSTER")) {
-    const int cl = atoi(force);
-    h->slice_cluster = built(cl) ? cl : 0;
-    return QD_OK;
-  }
-  const bool rf = built(SLICE_RF) || built(SLICE_RF2) || built(SLICE_RF4);
-  if (!rf && built(SLICE_AX)) {
-    h->slice_cluster = SLICE_AX;
-    return QD_OK;
-  }
-  // the choice depends on the shapes only: measured once per process and device
-  static std::mutex mu;
-  static std::map<std::tuple<int, int, int, int, int, int, int>, int> chosen;
-  int dev = 0;
-  cudaGetDevice(&dev);
-  const auto key = std::make_tuple(dev, h->n1, h->n2, h->nl, h->nruns, h->jrows,
-                                   h->d_run_k ? 1 : 0);
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = chosen.find(key);
-    if (it != chosen.end()) {
-      h->slice_cluster = it->second;
-      return QD_OK;
-    }
-  }
-  cudaEvent_t e0, e1;
-  CU(cudaEventCreate(&e0));
-  CU(cudaEventCreate(&e1));
-  LineParams p = line_params(h, true);
-  float best = 1e30f;
-  for (int cl : {0, 1, 2, 4, SLICE_RF, SLICE_RF2, SLICE_RF4, SLICE_RF4W}) {
-    if (rf ? !slice_is_rf(cl) || !built(cl) : cl > 0 && !built(cl)) continue;
-    p.cluster = cl;
-    bool ok = true;
-    for (int it = 0; it < 2 && ok; it++)
-      ok = run_lines(p, true, h->st) == cudaSuccess;
-    if (ok) ok = cudaEventRecord(e0, h->st) == cudaSuccess;
-    for (int it = 0; it < 5 && ok; it++)
-      ok = run_lines(p, true, h->st) == cudaSuccess;
-    if (ok) ok = cudaEventRecord(e1, h->st) == cudaSuccess;
-    if (ok) ok = cudaStreamSynchronize(h->st) == cudaSuccess;
-    float ms = 0.f;
-    if (ok) ok = cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess;
-    if (!ok) {                      // e.g. a cluster shape that cannot be scheduled
-      cudaGetLastError();
-      continue;
-    }
-    if (ms < best) { best = ms; h->slice_cluster = cl; }
-  }
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  CU(cudaMemsetAsync(h->d_lpsi, 0, sizeof(float2) * h->n12 * h->nl * h->nruns, h->st));
-  std::lock_guard<std::mutex> lock(mu);
-  chosen[key] = h->slice_cluster;
-  return QD_OK;
-}
-
 // Times `launch` (reps launches after one warm-up) on the handle's stream, ms
 // per launch; a negative value if a launch failed.
 template <typename F> float time_launches(qd_handle *h, F launch, int reps = 3)
@@ -638,6 +561,85 @@ template <typename F> float time_launches(qd_handle *h, F launch, int reps = 3)
   if (e0) cudaEventDestroy(e0);
   if (e1) cudaEventDestroy(e1);
   return ms;
+}
+
+// Choice of the l-space kernel.
+//   complex64, sizes compiled in: the register-FFT slice kernel on 1, 2 or 4
+//     CTAs per slice, timed on the handle's zero l-space buffer (a zero
+//     wavepacket stays zero), the choice kept for later handles of the shapes;
+//   sizes that k_axis_f32.cu / k_axis_f64.cu take: those (complex64, us a step,
+//     the best Stockham form -> k_axis_f32: 48 x 40 x 24 16.3 -> 14.7, 54 x 60 x 32
+//     25 -> 16, 144 x 120 x 64 52 -> 24, 200 x 180 x 40 93 -> 30, 8 runs of
+//     96 x 96 x 48 105 -> 45; FP64: k_axis_f64.cu);
+//   complex64 grids of few columns (n1 <= 32, or n1 <= 64 with n2 >= 256), whose
+//     column launch has one to four CTAs per slice for a long transform: those
+//     and the Stockham slice kernel on 1, 2 or 4 CTAs per slice, timed in steps
+//     (us a step, k_axis_f32 and the best Stockham form: 6 x 256 x 8 23.7 and 19.1,
+//     16 x 256 x 16 23.9 and 21.1, 16 x 400 x 16 26.8 and 25.3, 4 runs of
+//     64 x 256 x 8 43.3 and 41.7; but 24 x 60 x 16 15.9 and 19.1, 32 x 400 x 16 27.2
+//     and 33.5; 36 to 64 columns with n2 <= 240, or more columns: k_axis_f32 as fast
+//     within 3 % or faster on every grid that was timed);
+//   other grids: FP64 the split kernels; complex64 the split kernels or the
+//     Stockham slice kernel on 1, 2 or 4 CTAs per slice, timed likewise.
+// QD_SLICE_CLUSTER=0|1|2|4|8|9|10|11|12 forces a choice (0 the split kernels,
+// 1, 2, 4 the Stockham slice kernel, 8, 9, 10 the register-FFT kernel on 1, 2
+// and 4 CTAs, 11 its wide form, 12 the run-time register-FFT kernels; FP64 knows
+// 0 and 12 only).
+int tune_slice(qd_handle *h)
+{
+  const bool f32 = h->prec == QD_PREC_FP32;
+  h->slice_cluster = !f32 && axis_f64(h) ? SLICE_AX : 0;
+  if (!f32) return QD_OK;
+  auto built = [&](int cl) { return slice_cluster_ok(h->n1, h->n2, cl) != 0; };
+  if (const char *force = getenv("QD_SLICE_CLUSTER")) {
+    const int cl = atoi(force);
+    h->slice_cluster = built(cl) ? cl : 0;
+    return QD_OK;
+  }
+  const bool rf = built(SLICE_RF) || built(SLICE_RF2) || built(SLICE_RF4);
+  const bool ax = !rf && built(SLICE_AX);
+  const bool few_columns = h->n1 <= 32 || (h->n1 <= 64 && h->n2 >= 256);
+  if (ax && !few_columns) {
+    h->slice_cluster = SLICE_AX;
+    return QD_OK;
+  }
+  // the choice depends on the shapes only: measured once per process and device
+  static std::mutex mu;
+  static std::map<std::tuple<int, int, int, int, int, int, int>, int> chosen;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  const auto key = std::make_tuple(dev, h->n1, h->n2, h->nl, h->nruns, h->jrows,
+                                   h->d_run_k ? 1 : 0);
+  {
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = chosen.find(key);
+    if (it != chosen.end()) {
+      h->slice_cluster = it->second;
+      return QD_OK;
+    }
+  }
+  LineParams p = line_params(h, true);
+  const ColumnParams c = column_params(h);
+  float best = 1e30f;
+  for (int cl : {SLICE_AX, 0, 1, 2, 4, SLICE_RF, SLICE_RF2, SLICE_RF4, SLICE_RF4W}) {
+    if (rf ? !slice_is_rf(cl) : slice_is_rf(cl) || (ax && cl == 0)) continue;
+    if (cl > 0 && !built(cl)) continue;
+    p.cluster = cl;
+    // (a form that fails, such as a cluster shape that cannot be scheduled, gives no time)
+    const float ms = time_launches(h, [&] {
+      // few columns: a step, as the launches of k_axis_f32 overlap their neighbours and
+      // the Stockham kernel's does not (alone the wrong one was picked, by up to 8 % of a step)
+      cudaError_t e = cudaSuccess;
+      if (ax) e = h->use_tc ? launch_column_tc(h->tc, c, COL_MID, h->st)
+                            : launch_column<float>(c, COL_MID, h->st);
+      return e != cudaSuccess ? e : run_lines(p, true, h->st);
+    }, ax ? 20 : 5);
+    if (ms >= 0.f && ms < (ax ? 0.99f * best : best)) { best = ms; h->slice_cluster = cl; }
+  }
+  CU(cudaMemsetAsync(h->d_lpsi, 0, sizeof(float2) * h->n12 * h->nl * h->nruns, h->st));
+  std::lock_guard<std::mutex> lock(mu);
+  chosen[key] = h->slice_cluster;
+  return QD_OK;
 }
 
 // Autotuner of the flux-accumulation GEMM: each tile variant accumulates one

@@ -43,3 +43,19 @@ def test_description(fp64, ch, lines, column):
     import bench
     got = bench.describe_choice(ch, fp64)
     assert lines in got["l_space"] and column in got["column"], got
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n1,n2,nth,kinds", [
+    (6, 256, 8, (1, 2, 4)),             # 19.1 us a step against 23.6 on the run-time kernels
+    (12, 256, 8, (1, 2, 4)),            # 21.2 and 24.3
+    (40, 60, 16, (12,)), (96, 240, 8, (12,))])      # 16.8 and 21.2; never timed
+def test_grids_of_few_columns_are_timed(qdlib, n1, n2, nth, kinds):
+    from qd_b200 import Propagator
+    d = S.build_case("h+h2", n1, n2, nth, m=nth - 1, total_steps=1, n_energies=5,
+                     n_gradient_points=3)
+    d.options.precision = QD_PREC_FP32
+    with Propagator(d) as p:
+        ch = (C.c_int32 * 4)()
+        assert qdlib.qd_kernel_choice(p._h, ch) == 0
+    assert ch[0] in kinds
