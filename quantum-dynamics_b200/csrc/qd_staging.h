@@ -12,6 +12,7 @@
 #include <mutex>
 #include <thread>
 #include <vector>
+#include <sys/mman.h>
 #include <unistd.h>
 #ifdef __SSE2__
 #include <emmintrin.h>
@@ -144,10 +145,13 @@ class Staging {
   static constexpr size_t CHUNK = size_t(32) << 20;   // bytes per staging buffer
   static constexpr int NBUF = 4;
   static constexpr size_t LARGE = size_t(4) << 20;    // transfers from this size on use it
-  // results of the set-up calls from this size on: below, the copy threads cost more than
-  // they take off the faults of a fresh result array (a surface call with 1.2 MB 405 us
-  // staged, 260 not, with 1.3 MB 470 and 300)
-  static constexpr size_t FETCH = size_t(2) << 20;
+  // results of the set-up calls: staged from FETCH on where the array's pages are fresh,
+  // as the copy threads share their faults, and from FETCH_WARM on where they are in memory
+  // (a LEPS grid, us a call, plain and staged.  Fresh pages: 1.2 MB 260 and 405, 4.2 MB
+  // 1500 and 1230, 8.4 MB 2400 and 1900, 33.6 MB 7600 and 4600; in memory: 2.1 MB 190
+  // and 460, 8.4 MB 560 and 1440, 31.5 MB 1850 and 3500, 41.9 MB 2300 and 2700, 67 MB
+  // 3900 and 2800)
+  static constexpr size_t FETCH = size_t(2) << 20, FETCH_WARM = size_t(48) << 20;
 
   static Staging &get()
   {
@@ -313,7 +317,8 @@ class Staging {
   // the kernel leaves the staging buffers to other threads' copies
   cudaError_t fetch(void *dst, const void *src, size_t bytes)
   {
-    if (bytes < FETCH) return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
+    if (bytes < FETCH || (bytes < FETCH_WARM && in_memory(dst, bytes)))
+      return cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost);
     const cudaError_t e = cudaStreamSynchronize(nullptr);
     const Piece one{dst, src, bytes};
     return e == cudaSuccess ? download(&one, 1, nullptr, FETCH) : e;
@@ -321,6 +326,19 @@ class Staging {
 
  private:
   Staging() = default;
+  // most pages of [p, p + n) are in memory: 32 of them are looked at
+  static bool in_memory(const void *p, size_t n)
+  {
+    constexpr int SAMPLES = 32;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), at = reinterpret_cast<uintptr_t>(p);
+    int in = 0;
+    for (int i = 0; i < SAMPLES; i++) {
+      unsigned char v = 0;
+      if (mincore(reinterpret_cast<void *>((at + n / SAMPLES * i) & ~(page - 1)), 1, &v) == 0)
+        in += v & 1;
+    }
+    return 2 * in > SAMPLES;
+  }
   // the buffers, and the current device's events, exist (made on first use)
   bool ready()
   {

@@ -124,7 +124,27 @@ def test_fewer_worker_threads_than_asked_for(tmp_path, threads):
     int main() {
       const V a = ramp((size_t(5) << 20) / 8);
       V b(a.size());
-      CHECK(Staging::get().fetch(b.data(), a.data(), 8 * a.size()) == cudaSuccess);
+      CHECK(Staging::get().download(b.data(), a.data(), 8 * a.size(), nullptr) == cudaSuccess);
       CHECK(b == a && given <= %d && all_finite(a.data(), a.size()));
       return 0;
     }""" % (threads, threads), "-rdynamic", "-D_GNU_SOURCE")
+
+
+def test_results_into_warm_pages_are_not_staged(tmp_path):
+    # an array whose pages are in memory: a plain copy up to FETCH_WARM; a fresh mapping of
+    # the same size: staged
+    run(tmp_path, """
+    #include <sys/mman.h>
+    int main() {
+      Staging &s = Staging::get();
+      const size_t n = size_t(8) << 20;
+      const V a = ramp(n / 8);
+      V warm(n / 8);
+      CHECK(s.fetch(warm.data(), a.data(), n) == cudaSuccess && warm == a);
+      CHECK(s.fetch(warm.data() + 1, a.data(), n - 8) == cudaSuccess && warm[1] == a[0]);
+      CHECK(fake::pinned == 0);
+      double *f = (double *)mmap(nullptr, n, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+      CHECK(f != MAP_FAILED && s.fetch(f, a.data(), n) == cudaSuccess);
+      CHECK(std::equal(a.begin(), a.end(), f) && fake::pinned > 0);
+      return 0;
+    }""")
