@@ -1,6 +1,6 @@
 // k_axis_f32.cu -- the l-space part of one complex64 split-operator step for any
 // grid whose sizes are two groups of one or two radices (every even product of
-// 2, 3 and 5 from 6 to 256 but 8 and 162, some larger and some odd ones):
+// 2, 3 and 5 from 6 to 256 but 8 and 162, and some larger ones up to 800):
 //     psi_l <- Rot(dt/2) IFFT2 [exp(-i(T1+T2)dt)/(n1 n2)] FFT2 Rot(dt/2) psi_l
 // (evolution_dt, timeEvol.C:625-635; tables timeEvol.C:465-517).
 //

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(256) k_flux_phase(AccumParams p)
 // values, so that 16-byte accesses of a quarter-warp touch every bank group once.
 // Bound: FP64 tensor rate (37 TFLOP/s measured) and, in short chunks, reading and
 // writing phi and dphi (32-byte accesses).  250 steps of 241 energies on 8192
-// points (7.9 GFLOP, 250 MB): 398 us on plain FMAs, 278 so; of 150 energies on 3
+// points (7.9 GFLOP, 190 MB): 398 us on plain FMAs, 278 so; of 150 energies on 3
 // runs of 5400 points: 505, 377.  MG = 4 reads the history less often, MG = 2
 // wastes less of a last energy tile and fills the SMs better (the tuner times
 // both: 278 and 298, 425 and 377).  KT = 32: 311, 366.

@@ -580,7 +580,7 @@ cudaError_t launch_slice_rf(const LineParams &p, int cl, cudaStream_t s)
     if (p.n1 == 128 && p.n2 == 96) return launch_rf<128, 96, 256, 1>(p, s);
     if (p.n1 == 128 && p.n2 == 128) return launch_rf<128, 128, 512, 1>(p, s);
   } else if (cl == 2) {
-    // 64 x 64 x 40: 18.3 us a step on one CTA per slice, 15.0 on two (78 CTAs)
+    // 64 x 64 x 40: 19.3 us a step on one CTA per slice, 16.0 on two (78 CTAs)
     if (p.n1 == 64 && p.n2 == 64) return launch_rf<64, 64, 256, 2>(p, s);
     // one CTA per SM at most: 384 threads instead of 256 (128 x 96 x 64, one run: 18.1 us a
     // step against 24.1); more CTAs: two of 256 share an SM (two runs: 30.1 against 33.3)
